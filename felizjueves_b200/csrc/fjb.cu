@@ -1405,11 +1405,17 @@ void choose_rys(int mode, ClassRun &r) {
     if (r.rys32) r.grid_r32 = rgrid(true, r.ry32);
 }
 
-// The Rys rule's table, built once per process (rys_table.cpp).
-const std::vector<double> &rys_table_cached() {
-    static std::once_flag once;
-    static std::vector<double> t;
-    std::call_once(once, [] { t = rys_table(); });
+// The Rys rule's device tables, FP64 and FP32, built once per process
+// (rys_table.cpp).
+struct RysTables {
+    std::vector<double> t64;
+    std::vector<float> t32;
+};
+const RysTables &rys_tables_cached() {
+    static const RysTables t = [] {
+        const std::vector<double> f = rys_device_table(kRysDegF);
+        return RysTables{rys_device_table(kRysDegD), std::vector<float>(f.begin(), f.end())};
+    }();
     return t;
 }
 
@@ -1422,9 +1428,8 @@ int finish_create(std::unique_ptr<fjb_handle> &h, fjb_handle **out) {
     if (cudaSetDevice(device) != cudaSuccess) return fail(nullptr, FJB_E_CUDA, "cudaSetDevice failed");
     try {
         h->boys.upload(boys_table());
-        h->rys.upload(rys_table_cached());
-        const std::vector<double> &t = rys_table_cached();
-        h->rys32.upload(std::vector<float>(t.begin(), t.end()));
+        h->rys.upload(rys_tables_cached().t64);
+        h->rys32.upload(rys_tables_cached().t32);
         std::vector<int> off(h->basis.offsets), nc;
         for (auto &s : h->basis.shells) nc.push_back((s.l + 1) * (s.l + 2) / 2);
         h->sh_off.upload(off);

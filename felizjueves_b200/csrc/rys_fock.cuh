@@ -219,62 +219,42 @@ __host__ __device__ constexpr int rys_smem_budget(int minb) {
     return minb <= 1 ? kSmemBudgetDoubles : (233472 / minb - 1024 - 3072) / 8;
 }
 
-// One root of the n-point rule at T (rys_rule, one root's two series).
-template <int N>
-__device__ __forceinline__ void rule_root(int r, double T, const double *__restrict__ tab, double *x, double *w) {
+// One root of the n-point rule at T (rys_rule, one root's two series) from
+// the device table: a power's coefficients of x and of w are one vector load.
+template <int N, int DEG, typename R, typename R2>
+__device__ __forceinline__ void rule_series(int r, double T, const R *__restrict__ tab, R *x, R *w) {
     if (T < kRysTSwitch) {
         int i = (int)T;
         if (i > kRysNI - 1) i = kRysNI - 1;
-        const double u = 2.0 * (T - (double)i) - 1.0;  // kRysWidth = 1
-        const double *blk = tab + ((size_t)(N - 1) * kRysNI + i) * kRysBlock + (size_t)(2 * r) * (kRysDeg + 1);
-        double bx1 = 0.0, bx2 = 0.0, bw1 = 0.0, bw2 = 0.0;
-        const double u2 = 2.0 * u;
+        const R u = (R)(2.0 * (T - (double)i) - 1.0);  // kRysWidth = 1
+        const R2 *blk = reinterpret_cast<const R2 *>(tab + rys_device_at(DEG, N, i, 0, r));
+        R2 c[DEG + 1];
 #pragma unroll
-        for (int k = kRysDeg; k >= 1; --k) {
-            const double bx0 = u2 * bx1 - bx2 + __ldg(blk + k);
-            const double bw0 = u2 * bw1 - bw2 + __ldg(blk + kRysDeg + 1 + k);
-            bx2 = bx1;
-            bx1 = bx0;
-            bw2 = bw1;
-            bw1 = bw0;
+        for (int k = 0; k <= DEG; ++k) c[k] = __ldg(blk + k * N);
+        R px = c[DEG].x, pw = c[DEG].y;
+#pragma unroll
+        for (int k = DEG - 1; k >= 0; --k) {
+            px = px * u + c[k].x;
+            pw = pw * u + c[k].y;
         }
-        *x = u * bx1 - bx2 + __ldg(blk);
-        *w = u * bw1 - bw2 + __ldg(blk + kRysDeg + 1);
+        *x = px;
+        *w = pw;
     } else {
-        const double *a = tab + kRysAsym + (size_t)(N - 1) * kRysMaxN * 2;
-        *x = __ldg(a + 2 * r) / T;
-        *w = __ldg(a + 2 * r + 1) * (0.5 / sqrt(T));
+        const R *a = tab + rys_device_asym(DEG, N);
+        *x = (R)((double)__ldg(a + 2 * r) / T);
+        *w = (R)((double)__ldg(a + 2 * r + 1) * (0.5 / sqrt(T)));
     }
 }
-
-// The same root in FP32 from the table's FP32 copy (the routed path's FP32
-// tier): the interval and its local coordinate from T in FP64, the series
-// in FP32 (relative error about 1e-6, inside the tier's own).
+template <int N>
+__device__ __forceinline__ void rule_root(int r, double T, const double *__restrict__ tab, double *x, double *w) {
+    rule_series<N, kRysDegD, double, double2>(r, T, tab, x, w);
+}
+// The same root in FP32 from the FP32 table (the routed path's FP32 tier):
+// the interval and its local coordinate from T in FP64, the series in FP32
+// (relative error about 1e-7, inside the tier's own).
 template <int N>
 __device__ __forceinline__ void rule_root_f(int r, double T, const float *__restrict__ tab, float *x, float *w) {
-    if (T < kRysTSwitch) {
-        int i = (int)T;
-        if (i > kRysNI - 1) i = kRysNI - 1;
-        const float u = (float)(2.0 * (T - (double)i) - 1.0);
-        const float *blk = tab + ((size_t)(N - 1) * kRysNI + i) * kRysBlock + (size_t)(2 * r) * (kRysDeg + 1);
-        float bx1 = 0.f, bx2 = 0.f, bw1 = 0.f, bw2 = 0.f;
-        const float u2 = 2.f * u;
-#pragma unroll
-        for (int k = kRysDeg; k >= 1; --k) {
-            const float bx0 = u2 * bx1 - bx2 + __ldg(blk + k);
-            const float bw0 = u2 * bw1 - bw2 + __ldg(blk + kRysDeg + 1 + k);
-            bx2 = bx1;
-            bx1 = bx0;
-            bw2 = bw1;
-            bw1 = bw0;
-        }
-        *x = u * bx1 - bx2 + __ldg(blk);
-        *w = u * bw1 - bw2 + __ldg(blk + kRysDeg + 1);
-    } else {
-        const float *a = tab + kRysAsym + (size_t)(N - 1) * kRysMaxN * 2;
-        *x = (float)(__ldg(a + 2 * r) / T);
-        *w = (float)(__ldg(a + 2 * r + 1) * (0.5 / sqrt(T)));
-    }
+    rule_series<N, kRysDegF, float, float2>(r, T, tab, x, w);
 }
 
 // The HRR coefficient `idx` of side LY for separation sep (= A - B or C - D).

@@ -39,6 +39,24 @@ constexpr int kRysTableSize = kRysAsym + kRysMaxN * kRysMaxN * 2;
 // [n-1][root][s | v].  Built once, on the host.
 std::vector<double> rys_table();
 
+// The table as the kernels read it: the Chebyshev series cut at degree deg
+// and rewritten in powers of u, [n-1][interval][power k][root][x | w] at
+// rys_device_at, then the same (s, v) constants at rys_device_asym.  The
+// first dropped coefficient is below 5e-17 of the value at kRysDegD (FP64)
+// and 5e-10 at kRysDegF (FP32); the series fall off so fast that the powers'
+// coefficients cancel no digits.  A warp's lanes hold the roots of a few T:
+// with the roots side by side a power's loads are one 16-byte vector a lane
+// and n lanes share its lines, where the host order gave every lane two
+// lines of its own for each coefficient.
+constexpr int kRysDegD = 12, kRysDegF = 7;
+std::vector<double> rys_device_table(int deg);
+FJB_HD constexpr size_t rys_device_at(int deg, int n, int interval, int k, int r) {
+    return ((size_t)(n - 1) * kRysNI + interval) * ((deg + 1) * 2 * kRysMaxN) + (size_t)(k * n + r) * 2;
+}
+FJB_HD constexpr size_t rys_device_asym(int deg, int n) {
+    return (size_t)kRysMaxN * kRysNI * ((deg + 1) * 2 * kRysMaxN) + (size_t)(n - 1) * kRysMaxN * 2;
+}
+
 FJB_HD inline double rys_clenshaw(const double *c, double u) {
     double b1 = 0.0, b2 = 0.0;
     for (int k = kRysDeg; k >= 1; --k) {

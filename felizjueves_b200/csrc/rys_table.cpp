@@ -150,10 +150,9 @@ void rule_at(int n, LD T, const std::vector<LD> &gt, const std::vector<LD> &gu, 
     for (int i = 0; i < n; ++i) w[i] = mu0 * f[i] * f[i];
 }
 
-}  // namespace
-
-std::vector<double> rys_table() {
-    std::vector<double> tab(kRysTableSize, 0.0);
+// rys_table's layout in long double: the series before their rounding.
+std::vector<LD> rys_series() {
+    std::vector<LD> tab(kRysTableSize, 0.0L);
     std::vector<LD> gt, gu;
     gauss_legendre(kRysQuad, &gt, &gu);
     const int P = kRysDeg + 1;
@@ -166,7 +165,7 @@ std::vector<double> rys_table() {
                 rule_at(n, a + 0.5L * (uj + 1.0L) * (LD)kRysWidth, gt, gu, &xs[(size_t)j * kRysMaxN],
                         &ws[(size_t)j * kRysMaxN]);
             }
-            double *blk = tab.data() + ((size_t)(n - 1) * kRysNI + i) * kRysBlock;
+            LD *blk = tab.data() + ((size_t)(n - 1) * kRysNI + i) * kRysBlock;
             for (int r = 0; r < n; ++r)
                 for (int k = 0; k < P; ++k) {
                     LD cx = 0.0L, cw = 0.0L;
@@ -176,8 +175,8 @@ std::vector<double> rys_table() {
                         cw += ws[(size_t)j * kRysMaxN + r] * ck;
                     }
                     const LD s = (k == 0 ? 1.0L : 2.0L) / (LD)P;
-                    blk[(2 * r) * P + k] = (double)(cx * s);
-                    blk[(2 * r + 1) * P + k] = (double)(cw * s);
+                    blk[(2 * r) * P + k] = cx * s;
+                    blk[(2 * r + 1) * P + k] = cw * s;
                 }
         }
     // the asymptotic rule: generalised Gauss-Laguerre, alpha = -1/2
@@ -187,13 +186,44 @@ std::vector<double> rys_table() {
         for (int k = 1; k < n; ++k) J[(size_t)(k - 1) * n + k] = J[(size_t)k * n + k - 1] = sqrtl((LD)k * ((LD)k - 0.5L));
         std::vector<LD> s(n), f(n);
         jacobi_eig(n, J, s.data(), f.data());
-        double *a = tab.data() + kRysAsym + (size_t)(n - 1) * kRysMaxN * 2;
+        LD *a = tab.data() + kRysAsym + (size_t)(n - 1) * kRysMaxN * 2;
         for (int r = 0; r < n; ++r) {
-            a[2 * r] = (double)s[r];
-            a[2 * r + 1] = (double)(sqrtl(kPiL) * f[r] * f[r]);
+            a[2 * r] = s[r];
+            a[2 * r + 1] = sqrtl(kPiL) * f[r] * f[r];
         }
     }
     return tab;
+}
+
+}  // namespace
+
+std::vector<double> rys_table() {
+    const std::vector<LD> s = rys_series();
+    return std::vector<double>(s.begin(), s.end());
+}
+
+std::vector<double> rys_device_table(int deg) {
+    static const std::vector<LD> h = rys_series();
+    std::vector<double> d(rys_device_asym(deg, 1) + kRysMaxN * kRysMaxN * 2, 0.0);
+    std::transform(h.begin() + kRysAsym, h.end(), d.begin() + rys_device_asym(deg, 1), [](LD v) { return (double)v; });
+    // T_k in powers of u
+    std::vector<std::vector<long double>> T(deg + 1, std::vector<long double>(deg + 1, 0.0L));
+    T[0][0] = 1.0L;
+    if (deg > 0) T[1][1] = 1.0L;
+    for (int k = 2; k <= deg; ++k)
+        for (int j = 0; j <= k; ++j) T[k][j] = (j ? 2.0L * T[k - 1][j - 1] : 0.0L) - T[k - 2][j];
+    for (int n = 1; n <= kRysMaxN; ++n)
+        for (int i = 0; i < kRysNI; ++i) {
+            const LD *blk = h.data() + ((size_t)(n - 1) * kRysNI + i) * kRysBlock;
+            for (int r = 0; r < n; ++r)
+                for (int c = 0; c < 2; ++c)
+                    for (int j = 0; j <= deg; ++j) {
+                        long double v = 0.0L;
+                        for (int k = j; k <= deg; ++k) v += blk[(2 * r + c) * (kRysDeg + 1) + k] * T[k][j];
+                        d[rys_device_at(deg, n, i, j, r) + c] = (double)v;
+                    }
+        }
+    return d;
 }
 
 }  // namespace fjb
