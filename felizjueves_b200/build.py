@@ -18,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -27,7 +28,9 @@ LIB = os.path.join(OUT_DIR, "libfjb.so")
 REPO = os.path.dirname(HERE)
 
 CU_SOURCES = ["fjb.cu", "fock_compiled.cu", "router.cu", "jengine.cu", "onee.cu", "rys_fock.cu",
-              "rys_fock64.cu", "rys_fock32.cu", "df_mm.cu", "df_eri3.cu"]
+              "rys_fock64.cu", "rys_fock32.cu", "df_mm.cu", "df_eri3.cu", "rys_warp.cu"]
+# rys_warp_inst.cu, once per bra class and precision (rys_warp.h's lists)
+RYS_WARP_PARTS = [(p, f) for p in ("SD", "SF", "SP", "PP", "PD", "DD") for f in (0, 1)]
 CPP_SOURCES = ["plan.cpp", "hgp_tables.cpp", "boys_table.cpp", "scatter.cpp", "rys_table.cpp", "hjk_plan.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -84,20 +87,25 @@ def build(force: bool = False, verbose: bool = False) -> str:
         obj = os.path.join(OUT_DIR, src + ".o")
         jobs.append(([cc, *common, *ARCH, "-lineinfo", "--fmad=true", "-c",
                       os.path.join(CSRC, src), "-o", obj], obj))
-    procs = []
-    for cmd, obj in jobs:
+    for part, fp32 in RYS_WARP_PARTS:
+        obj = os.path.join(OUT_DIR, f"rys_warp_{part}_{32 if fp32 else 64}.o")
+        jobs.append(([cc, *common, *ARCH, "-lineinfo", "--fmad=true", f"-DFJB_RW_PART=FJB_RW_{part}",
+                      f"-DFJB_RW_FP32={fp32}", "-c", os.path.join(CSRC, "rys_warp_inst.cu"), "-o", obj], obj))
+
+    def compile_one(job):
+        cmd, _ = job
         if verbose:
             print(" ".join(cmd), flush=True)
-        procs.append((subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.PIPE,
-                                       text=True), cmd, obj))
+        return subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True)
+
     failed = None
-    for p, cmd, obj in procs:
-        out, err = p.communicate()
-        if verbose or p.returncode:
-            sys.stdout.write(out)
-            sys.stderr.write(err)
-        if p.returncode and failed is None:
-            failed = cmd
+    with ThreadPoolExecutor(max_workers=max(8, os.cpu_count() or 1)) as pool:
+        for (cmd, _), r in zip(jobs, pool.map(compile_one, jobs)):
+            if verbose or r.returncode:
+                sys.stdout.write(r.stdout)
+                sys.stderr.write(r.stderr)
+            if r.returncode and failed is None:
+                failed = cmd
     if failed:
         raise RuntimeError(f"build step failed: {' '.join(failed[:4])} ...")
     objs = [obj for _, obj in jobs]

@@ -30,6 +30,7 @@
 #include "scatter.h"
 #include "router.cuh"
 #include "rys_fock.cuh"
+#include "rys_warp.h"
 #include "df_eri3.cuh"
 
 namespace fjb {
@@ -905,6 +906,9 @@ struct ClassRun {
     RysDev ry64{}, ry32{};
     int grid_r64 = 0, grid_r32 = 0;
     const double *rys_tab = nullptr;
+    // the warp-autonomous Rys kernel (rys_warp.cuh), when it takes the class
+    bool warp64 = false, warp32 = false;
+    int grid_w64 = 0, grid_w32 = 0;
     const float *rys_tab32 = nullptr;
     ClassDev dev32;  // the FP32 interpreter's layout (routed builds of classes without has32)
     int unit0 = 0, n_units = 0;
@@ -953,6 +957,11 @@ int run_grid(const ClassRun &r);
 // else the interpreter (which alone serves the atomics-free build's slots).
 cudaError_t launch_run(const ClassRun &r, cudaStream_t st, const KArgs &a) {
     if (r.rys64 && !a.W) {
+    if (r.warp64 && !a.W) {
+        KArgs ar = a;
+        ar.rys_tab = r.rys_tab;
+        return rys_warp_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, false, r.grid_w64, st, ar);
+    }
         KArgs ar = a;
         ar.Y = r.ry64;
         ar.rys_tab = r.rys_tab;
@@ -967,6 +976,11 @@ cudaError_t launch_run(const ClassRun &r, cudaStream_t st, const KArgs &a) {
 // the Rys kernel in FP32, else the interpreter in FP32 with its own layout.
 cudaError_t launch_run32(const ClassRun &r, cudaStream_t st, const KArgs &a) {
     if (r.has32) return launch_compiled(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid32, st, a);
+    if (r.warp32 && !a.W) {
+        KArgs ar = a;
+        ar.rys_tab32 = r.rys_tab32;
+        return rys_warp_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid_w32, st, ar);
+    }
     if (r.rys32 && !a.W) {
         KArgs ar = a;
         ar.Y = r.ry32;
@@ -1387,15 +1401,15 @@ int append_shells(fjb_handle *h, const fjb_basis *b, int max_l) {
 // Device staging common to every handle: the Boys table, shell offsets and
 // sizes, the build events.
 // Which kernels a class run's units take from the Rys kernel: mode 0 none;
-// 1 the classes without an FP64 register body, and those with one where the
-// Rys kernel is the faster (rys_preferred); 2 every class it has.  FP32:
-// the classes without an FP32 register body (modes 1 and 2).
+// 0 none; 1 the classes without an FP64 (FP32) register body and those where
+// the Rys kernel is the faster; 2 every class it has.  Bras of at most 32
+// Cartesians run on the warp kernel (rys_warp.cuh), the longer ones on the
+// CTA kernel (rys_fock.cuh).
 void choose_rys(int mode, ClassRun &r) {
     const int la = r.dev.la, lb = r.dev.lb, lc = r.dev.lc, ld = r.dev.ld;
-    const bool take64 = mode >= 1 && ((!r.compiled && rys_available(la, lb, lc, ld, false)) ||
-                                      (rys_extra(la, lb, lc, ld) && (mode == 2 || rys_preferred(la, lb, lc, ld))));
-    r.rys64 = take64 && rys_layout(la, lb, lc, ld, r.max_kab, r.max_kcd, false, kSmemBudgetDoubles, &r.ry64);
-    r.rys32 = mode >= 1 && !r.has32 && rys_available(la, lb, lc, ld, true) &&
+    r.rys64 = mode >= 1 && rys_available(la, lb, lc, ld) &&
+              rys_layout(la, lb, lc, ld, r.max_kab, r.max_kcd, false, kSmemBudgetDoubles, &r.ry64);
+    r.rys32 = mode >= 1 && rys_available(la, lb, lc, ld) &&
               rys_layout(la, lb, lc, ld, r.max_kab, r.max_kcd, true, kSmemBudgetDoubles, &r.ry32);
     const auto rgrid = [&](bool fp32, const RysDev &d) {
         const int per_sm = std::max(1, rys_blocks_per_sm(la, lb, lc, ld, fp32, d));
@@ -1421,6 +1435,18 @@ const RysTables &rys_tables_cached() {
 
 int finish_create(std::unique_ptr<fjb_handle> &h, fjb_handle **out) {
     const int device = h->device;
+    const auto wgrid = [&](bool fp32) {
+        const int64_t most = (int64_t)r.n_units * kKetChunk;  // a unit makes at most one item a ket
+        const int per_sm = std::max(1, rys_warp_blocks_per_sm(la, lb, lc, ld, fp32));
+        return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
+    };
+    const auto wtake = [&](bool fp32) {
+        return mode >= 1 && rys_warp_available(la, lb, lc, ld) && (mode == 2 || rys_warp_preferred(la, lb, lc, ld, fp32));
+    };
+    r.warp64 = wtake(false);
+    r.warp32 = wtake(true);
+    if (r.warp64) r.grid_w64 = wgrid(false);
+    if (r.warp32) r.grid_w32 = wgrid(true);
     if (device < 0) {  // host-only handle: plans and exports, no builds
         *out = h.release();
         return FJB_OK;
@@ -3353,7 +3379,7 @@ int fjb_batch_create(fjb_batch **out, fjb_handle *const *handles, int n) {
         choose_rys(1, r);
         r.grid = run_grid(r);
         r.grid32 = run_grid32(r);
-        if (!r.compiled && !r.rys64)
+        if (!r.compiled && !r.rys64 && !r.warp64)
             return bfail(nullptr, FJB_E_LIMIT, "fjb_batch_create: a class has neither a register nor a Rys kernel");
         cudaEvent_t e0, e1;
         if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
@@ -3421,7 +3447,7 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
         a.mols = b->ctx.p;
         a.launch_mol = b->launch_mol.p;
         if (routed) {
-            if (!r.has32 && !r.rys32)
+            if (!r.has32 && !r.rys32 && !r.warp32)
                 return bfail(b, FJB_E_LIMIT, "fjb_batch_build: a class has no FP32 kernel for routed units");
             int *l32 = b->route_list.p + r.unit0;
             int *l64 = b->route_list.p + b->n_units + r.unit0;

@@ -210,20 +210,20 @@ __device__ __forceinline__ void quartet_compiled(const KArgs &A, const MolCtx &M
 #pragma unroll
     for (int kk = 0; kk < NC; ++kk)
 #pragma unroll
-        for (int l = 0; l < ND; ++l) atomicAdd(M.Jp + (size_t)(oc + kk) * n_ao + od + l, w2 * jcd[kk * ND + l]);
+        for (int l = 0; l < ND; ++l) red_add(M.Jp + (size_t)(oc + kk) * n_ao + od + l, w2 * jcd[kk * ND + l]);
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
 #pragma unroll
-        for (int kk = 0; kk < NC; ++kk) atomicAdd(M.Kp + (size_t)(oa + i) * n_ao + oc + kk, deg * kac[i * NC + kk]);
+        for (int kk = 0; kk < NC; ++kk) red_add(M.Kp + (size_t)(oa + i) * n_ao + oc + kk, deg * kac[i * NC + kk]);
 #pragma unroll
-        for (int l = 0; l < ND; ++l) atomicAdd(M.Kp + (size_t)(oa + i) * n_ao + od + l, deg * kad[i * ND + l]);
+        for (int l = 0; l < ND; ++l) red_add(M.Kp + (size_t)(oa + i) * n_ao + od + l, deg * kad[i * ND + l]);
     }
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
 #pragma unroll
-        for (int kk = 0; kk < NC; ++kk) atomicAdd(M.Kp + (size_t)(ob + j) * n_ao + oc + kk, deg * kbc[j * NC + kk]);
+        for (int kk = 0; kk < NC; ++kk) red_add(M.Kp + (size_t)(ob + j) * n_ao + oc + kk, deg * kbc[j * NC + kk]);
 #pragma unroll
-        for (int l = 0; l < ND; ++l) atomicAdd(M.Kp + (size_t)(ob + j) * n_ao + od + l, deg * kbd[j * ND + l]);
+        for (int l = 0; l < ND; ++l) red_add(M.Kp + (size_t)(ob + j) * n_ao + od + l, deg * kbd[j * ND + l]);
     }
 }
 
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(128) hgp_compiled_kernel(const KArgs A) {
             if (A.W) {
                 if (lane == 0) A.wab[A.wab_off[u] + t] = v;  // the unit's partial, reduced in unit order
             } else if (lane == 0 && v != 0.0) {
-                atomicAdd(M.Jp + (size_t)(bra.ao_a + t / NB) * M.n_ao + bra.ao_b + t % NB, v);
+                red_add(M.Jp + (size_t)(bra.ao_a + t / NB) * M.n_ao + bra.ao_b + t % NB, v);
             }
         }
     }

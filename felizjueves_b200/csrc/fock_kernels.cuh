@@ -71,6 +71,13 @@ struct KArgs {
     const int32_t *launch_mol;
 };
 
+// *p += v in global memory, no value returned.  The accumulators' pointers come
+// out of MolCtx as generic ones, for which atomicAdd is a returning ATOM; this
+// is the plain reduction.
+__device__ __forceinline__ void red_add(double *p, double v) {
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
+}
+
 __device__ __forceinline__ MolCtx mol_of(const KArgs &A, int launch) {
     if (A.mols) return A.mols[A.launch_mol[launch]];
     return MolCtx{A.D, A.Dsh, A.Jp, A.Kp, A.n_ao, A.n_sh};

@@ -43,35 +43,16 @@
 #include "fock_kernels.cuh"
 #include "rys_rule.h"
 
-// The classes the Rys kernel takes: in FP64 every class whose HGP program
-// does not fit the register path (the shared-memory interpreter's classes),
-// in FP32 every class without an FP32 register body.
-#define FJB_RYS64_CLASSES(X)                                                                            \
-    X(0, 1, 2, 3) X(0, 1, 3, 3) X(0, 2, 1, 3) X(0, 2, 2, 2) X(0, 2, 2, 3) X(0, 2, 3, 3) X(0, 3, 0, 3)    \
-    X(0, 3, 1, 2) X(0, 3, 1, 3) X(0, 3, 2, 2) X(0, 3, 2, 3) X(0, 3, 3, 3) X(1, 1, 1, 3) X(1, 1, 2, 2)    \
-    X(1, 1, 2, 3) X(1, 1, 3, 3) X(1, 2, 1, 2) X(1, 2, 1, 3) X(1, 2, 2, 2) X(1, 2, 2, 3) X(1, 2, 3, 3)    \
-    X(1, 3, 1, 3) X(1, 3, 2, 2) X(1, 3, 2, 3) X(1, 3, 3, 3) X(2, 2, 2, 2) X(2, 2, 2, 3) X(2, 2, 3, 3)    \
-    X(2, 3, 2, 3) X(2, 3, 3, 3) X(3, 3, 3, 3)
-// Classes the register kernel also has in FP64, where the Rys kernel can
-// take them instead (fjb_set_rys mode 2, and the classes rys_preferred names)
-#define FJB_RYS64_EXTRA_CLASSES(X)                                                                      \
-    X(0, 0, 0, 1) X(0, 1, 0, 1) X(0, 1, 0, 2) X(0, 1, 0, 3) X(0, 1, 1, 1) X(0, 1, 1, 2) X(0, 1, 1, 3)    \
-    X(0, 1, 2, 2) X(0, 2, 0, 3) X(0, 2, 1, 1) X(0, 2, 1, 2) X(0, 3, 1, 1) X(1, 1, 1, 2)
-#define FJB_RYS32_CLASSES(X)                                                                            \
-    X(0, 2, 2, 3) X(0, 2, 3, 3) X(0, 3, 1, 3) X(0, 3, 2, 2) X(0, 3, 2, 3) X(0, 3, 3, 3) X(1, 1, 2, 3)    \
-    X(1, 1, 3, 3) X(1, 2, 1, 3) X(1, 2, 2, 2) X(1, 2, 2, 3) X(1, 2, 3, 3) X(1, 3, 1, 3) X(1, 3, 2, 2)    \
-    X(1, 3, 2, 3) X(1, 3, 3, 3) X(2, 2, 2, 2) X(2, 2, 2, 3) X(2, 2, 3, 3) X(2, 3, 2, 3) X(2, 3, 3, 3)    \
-    X(3, 3, 3, 3)
+// The classes this kernel takes, FP64 and FP32: the bras whose row of
+// Cartesians is longer than a warp (pf, df, ff).
+#define FJB_RYS_CLASSES(X)                                                                           \
+    X(1, 3, 1, 3) X(1, 3, 2, 2) X(1, 3, 2, 3) X(1, 3, 3, 3) X(2, 3, 2, 3) X(2, 3, 3, 3) X(3, 3, 3, 3)
 
 namespace fjb {
 
 
 // host side (rys_fock.cu)
-bool rys_available(int la, int lb, int lc, int ld, bool fp32);
-// FP64 classes that have a register-path body too: whether the Rys kernel
-// is the faster of the two (measured on the 64-atom cluster)
-bool rys_extra(int la, int lb, int lc, int ld);
-bool rys_preferred(int la, int lb, int lc, int ld);
+bool rys_available(int la, int lb, int lc, int ld);
 // The carve-up of a class's kernel for bra and ket degrees up to max_kab,
 // max_kcd within `budget` doubles of shared memory: kets per group G from
 // the CTA width, then the largest table chunk that fits.  false if none.
@@ -602,7 +583,7 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
                     const int c = o / ND, d = o - c * ND;
 #pragma unroll
                     for (int ab = 0; ab < NAB; ++ab) acc2 += Dab[ab] * (double)Y[ab * YS + o];
-                    atomicAdd(M.Jp + (size_t)(oc + c) * n_ao + od + d, 2.0 * deg * acc2);
+                    red_add(M.Jp + (size_t)(oc + c) * n_ao + od + d, 2.0 * deg * acc2);
                 } else if (o < NCD + NA * NC) {
                     const int r = o - NCD, a = r / NC, c = r - a * NC;
                     const double *dbd = dk + NCD + NA * NC + NA * ND + NB * NC;
@@ -610,7 +591,7 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
                     for (int b = 0; b < NB; ++b)
 #pragma unroll
                         for (int d = 0; d < ND; ++d) acc2 += dbd[b * ND + d] * (double)Y[(a * NB + b) * YS + c * ND + d];
-                    atomicAdd(M.Kp + (size_t)(oa + a) * n_ao + oc + c, deg * acc2);
+                    red_add(M.Kp + (size_t)(oa + a) * n_ao + oc + c, deg * acc2);
                 } else if (o < NCD + NA * NC + NA * ND) {
                     const int r = o - NCD - NA * NC, a = r / ND, d = r - a * ND;
                     const double *dbc = dk + NCD + NA * NC + NA * ND;
@@ -618,7 +599,7 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
                     for (int b = 0; b < NB; ++b)
 #pragma unroll
                         for (int c = 0; c < NC; ++c) acc2 += dbc[b * NC + c] * (double)Y[(a * NB + b) * YS + c * ND + d];
-                    atomicAdd(M.Kp + (size_t)(oa + a) * n_ao + od + d, deg * acc2);
+                    red_add(M.Kp + (size_t)(oa + a) * n_ao + od + d, deg * acc2);
                 } else if (o < NCD + NA * NC + NA * ND + NB * NC) {
                     const int r = o - NCD - NA * NC - NA * ND, b = r / NC, c = r - b * NC;
                     const double *dad = dk + NCD + NA * NC;
@@ -626,7 +607,7 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
                     for (int a = 0; a < NA; ++a)
 #pragma unroll
                         for (int d = 0; d < ND; ++d) acc2 += dad[a * ND + d] * (double)Y[(a * NB + b) * YS + c * ND + d];
-                    atomicAdd(M.Kp + (size_t)(ob + b) * n_ao + oc + c, deg * acc2);
+                    red_add(M.Kp + (size_t)(ob + b) * n_ao + oc + c, deg * acc2);
                 } else {
                     const int r = o - NCD - NA * NC - NA * ND - NB * NC, b = r / ND, d = r - b * ND;
                     const double *dac = dk + NCD;
@@ -634,7 +615,7 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
                     for (int a = 0; a < NA; ++a)
 #pragma unroll
                         for (int c = 0; c < NC; ++c) acc2 += dac[a * NC + c] * (double)Y[(a * NB + b) * YS + c * ND + d];
-                    atomicAdd(M.Kp + (size_t)(ob + b) * n_ao + od + d, deg * acc2);
+                    red_add(M.Kp + (size_t)(ob + b) * n_ao + od + d, deg * acc2);
                 }
             }
             __syncthreads();

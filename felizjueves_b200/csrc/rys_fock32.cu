@@ -1,5 +1,5 @@
-// rys_fock32.cu -- the Rys Fock kernel instantiated for its FP32 classes
-// (FJB_RYS32_CLASSES, rys_fock.cuh); compiled apart from the other precision so
+// rys_fock32.cu -- the Rys Fock kernel instantiated for its classes in FP32
+// (FJB_RYS_CLASSES, rys_fock.cuh); compiled apart from the other precision so
 // the two build in parallel.
 #include "rys_fock.cuh"
 
@@ -8,7 +8,7 @@ namespace fjb {
 int rys_blocks_per_sm32(int la, int lb, int lc, int ld, const RysDev &d) {
 #define FJB_X(a, b, c, e) \
     if (la == a && lb == b && lc == c && ld == e) return RysOne<a, b, c, e, float>::occupancy(d);
-    FJB_RYS32_CLASSES(FJB_X)
+    FJB_RYS_CLASSES(FJB_X)
 #undef FJB_X
     return 0;
 }
@@ -16,7 +16,7 @@ int rys_blocks_per_sm32(int la, int lb, int lc, int ld, const RysDev &d) {
 cudaError_t rys_launch32(int la, int lb, int lc, int ld, int grid, cudaStream_t st, const KArgs &a) {
 #define FJB_X(a_, b_, c_, e_) \
     if (la == a_ && lb == b_ && lc == c_ && ld == e_) return RysOne<a_, b_, c_, e_, float>::launch(grid, st, a);
-    FJB_RYS32_CLASSES(FJB_X)
+    FJB_RYS_CLASSES(FJB_X)
 #undef FJB_X
     return cudaErrorInvalidValue;
 }

@@ -1,0 +1,114 @@
+"""The warp-autonomous Rys kernel (rys_warp.cuh) at the sizes where its split
+can go wrong: fewer kets than a group (one atom), units cut into slices (small
+systems) and not (a system whose units outnumber the grid), every class it is
+built for (set_rys(2)), and contraction degrees that leave ragged table rounds
+-- against the register kernel and the HGP interpreter (set_rys(0)), whose
+boundary and transfers are other code, at the plain FP64 bar."""
+
+import numpy as np
+import pytest
+
+from felizjueves_b200 import configs
+from felizjueves_b200.fock import FockEngine
+from felizjueves_b200.shell import Basis, Shell, primitive_norm
+
+pytestmark = pytest.mark.gpu
+
+
+def _ragged(seed):
+    """Three centres with s, p, d, f shells of degrees 1, 2, 5 and 7."""
+    rng = np.random.default_rng(seed)
+    shells = []
+    for c in rng.uniform(0.0, 4.0, (3, 3)):
+        for l, deg in ((0, 7), (0, 1), (1, 5), (1, 1), (2, 2), (2, 1), (3, 1), (3, 2)):
+            ex = [0.25 * 2.7 ** k * (1 + 0.1 * l) for k in range(deg)]
+            shells.append(Shell(l, tuple(map(float, c)), ex, [primitive_norm(l, e) / deg for e in ex]))
+    B = Basis(tuple(shells))
+    return B, configs.random_density(rng, B.n_ao, 6)
+
+
+def _system(name):
+    if name == "ragged":
+        return _ragged(3)
+    w = configs.cluster(int(name), 5 + int(name))
+    return w.basis, w.D
+
+
+@pytest.mark.parametrize("name", ["1", "2", "7", "ragged"])
+def test_warp_kernel_matches_other_engines(cuda, lib_built, name):
+    basis, D = _system(name)
+    eng = FockEngine(basis)
+    eng.plan(D, 1e-12, 4, export=False)
+    out = {}
+    for mode in (0, 1, 2):
+        eng.set_rys(mode)
+        out[mode] = (eng.build_host(D), sum(s["computed"] for s in eng.launch_stats()))
+    scale = max(1.0, np.abs(out[0][0][0]).max() / 100.0)  # 1e-13 of the largest element above 100
+    for mode in (1, 2):
+        assert out[mode][1] == out[0][1]  # every quartet once, slices or not
+        for a, b in zip(out[mode][0], out[0][0]):
+            assert np.abs(a - b).max() <= 1e-11 * scale
+
+
+@pytest.mark.parametrize("name", ["1", "7", "ragged"])
+def test_warp_kernel_fp32_tier(cuda, lib_built, name):
+    """Every unit in FP32, unchecked, mode 2: FP32 accuracy relative to G."""
+    from felizjueves_b200 import _lib
+    basis, D = _system(name)
+    eng = FockEngine(basis)
+    eng.plan(D, 1e-12, 4, export=False)
+    G = eng.build_host(D)[2]
+    eng.set_rys(2)
+    eng.set_route_check(0.0)
+    G32 = eng.build_host(D, precision=_lib.FJB_ROUTED, threshold=1e30)[2]
+    assert 0.0 < np.abs(G32 - G).max() <= 1e-5 * np.abs(G).max()
+
+
+@pytest.mark.parametrize("precision,threshold", [(0, 0.0), (1, 1e-9)])
+def test_overlapped_build_order(cuda, lib_built, precision, threshold):
+    """A small build forks its class launches onto side streams: D written
+    just before it on the caller's stream is the D it reads, its outputs are
+    ready for that stream, and the captured graph gives the same."""
+    import torch
+    w = configs.cluster(4, 9)
+    eng = FockEngine(w.basis)
+    eng.plan(w.D, w.tau, w.n_mag, export=False)
+    ref = [torch.tensor(m, device=cuda) for m in eng.build_host(w.D)]
+    D0 = torch.tensor(w.D, device=cuda)
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for graph in (False, True, False):
+        D, outs = torch.zeros_like(D0), [torch.zeros_like(D0) for _ in range(3)]
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st):
+            for _ in range(3):
+                D.zero_()
+                D.add_(D0)
+                eng.build(D, J=outs[0], K=outs[1], G=outs[2], precision=precision, threshold=threshold, graph=graph)
+                got = [o.clone() for o in outs]
+                for o in outs:
+                    o.fill_(float("nan"))
+        st.synchronize()
+        for a, b in zip(got, ref):
+            assert float((a - b).abs().max()) <= (1e-11 if precision == 0 else 1e-8)
+
+
+@pytest.mark.parametrize("atoms", [1, 2, 5])
+def test_j_engine_orders_and_reproduces(cuda, lib_built, oracle_lib, atoms):
+    """The J-engine's Rys classes with fewer kets than a warp's step (one
+    atom: one ff record) and ragged last steps, against the oracle; and the
+    same bits on every build (one writer an element, fixed order)."""
+    import torch
+    w = configs.cluster(atoms, 3)
+    eng = FockEngine(w.basis)
+    D = torch.tensor(w.D, device=cuda)
+    J = eng.coulomb(D, tau=0.0).clone()
+    again = eng.coulomb(D, tau=0.0).clone()
+    torch.cuda.synchronize()
+    assert torch.equal(J, again)
+    if atoms < 5:
+        Jo, _ = oracle_lib.jk(oracle_lib.OracleBasis.of(w.basis), w.D)
+        assert np.abs(J.cpu().numpy() - Jo).max() <= 1e-11
+    else:
+        eng.plan(w.D, 0.0, 4, export=False)
+        assert float((J - eng.build(D)[0]).abs().max()) <= 1e-11
