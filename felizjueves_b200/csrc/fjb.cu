@@ -31,6 +31,7 @@
 #include "router.cuh"
 #include "rys_fock.cuh"
 #include "rys_warp.h"
+#include "side_streams.h"
 #include "df_eri3.cuh"
 
 namespace fjb {
@@ -995,9 +996,25 @@ cudaError_t launch_run32(const ClassRun &r, cudaStream_t st, const KArgs &a) {
 
 }  // namespace
 
+// Builds of at most this many work units overlap their class launches.
+constexpr int kOverlapUnits = 1 << 22;
+
+// Whether a build on st overlaps: it is small enough, and its side streams
+// are there (made on first use, but not while st is being captured).
+cudaError_t use_side_streams(SideStreams &side, int n_units, bool capturing, bool *use) {
+    *use = n_units <= kOverlapUnits;
+    if (!*use || side.ready) return cudaSuccess;
+    if (capturing) {
+        *use = false;
+        return cudaSuccess;
+    }
+    return side.ensure();
+}
+
 struct fjb_handle {
     int device = 0;
     HostBasis basis;
+    SideStreams side;
     fjb::JEngine *jeng = nullptr;  // the J-engine, built on first use
     fjb::OneElectron *onee = nullptr;  // the one-electron shell pairs, built on first use
     std::vector<fjb::PairBounds> pair_bounds;  // the plan's D-independent pair bounds, computed once
@@ -1413,7 +1430,8 @@ void choose_rys(int mode, ClassRun &r) {
               rys_layout(la, lb, lc, ld, r.max_kab, r.max_kcd, true, kSmemBudgetDoubles, &r.ry32);
     const auto rgrid = [&](bool fp32, const RysDev &d) {
         const int per_sm = std::max(1, rys_blocks_per_sm(la, lb, lc, ld, fp32, d));
-        return std::max(1, std::min(r.n_units, per_sm * sm_count()));
+        const int64_t most = (int64_t)r.n_units * ((kKetChunk + d.group - 1) / d.group);  // a slice a group
+        return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
     };
     if (r.rys64) r.grid_r64 = rgrid(false, r.ry64);
     if (r.rys32) r.grid_r32 = rgrid(true, r.ry32);
@@ -1851,9 +1869,16 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
     CUDA_OK(h, cudaStreamIsCapturing(st, &cap));
     const unsigned ev_flags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     CUDA_OK(h, cudaEventRecordWithFlags(h->ev0, st, ev_flags));
-    for (size_t ri = 0; ri < h->runs.size(); ++ri) {
+    bool overlap = false;
+    CUDA_OK(h, use_side_streams(h->side, h->n_units, cap == cudaStreamCaptureStatusActive, &overlap));
+    overlap = overlap && !scatter;
+    if (overlap) CUDA_OK(h, h->side.fork(st));
+    // the large classes first: their kernels are the longest
+    for (size_t rj = 0; rj < h->runs.size(); ++rj) {
+        const size_t ri = h->runs.size() - 1 - rj;
         const ClassRun &r = h->runs[ri];
-        CUDA_OK(h, cudaEventRecordWithFlags(h->cev[ri].first, st, ev_flags));
+        const cudaStream_t cs = overlap ? h->side.s[rj % SideStreams::kN] : st;
+        CUDA_OK(h, cudaEventRecordWithFlags(h->cev[ri].first, cs, ev_flags));
         KArgs a{};
         a.computed = h->computed.p;
         a.C = r.dev;
@@ -1887,13 +1912,13 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
             const int stride = check ? h->check_stride : 0;
             const int rgrid = std::max(1, std::min((r.n_units + 3) / 4, 16 * sm_count()));
             if (h->router_on && r.dev.la + r.dev.lb + r.dev.lc + r.dev.ld >= h->router_min_l)
-                route_units_mlp_kernel<<<rgrid, 128, 0, st>>>(
+                route_units_mlp_kernel<<<rgrid, 128, 0, cs>>>(
                     h->units.p, r.unit0, r.n_units, h->launches.p, h->pairs.p, h->prims.p, h->Dsh.p, nsh,
                     h->plan.tau, route, h->router_p.p, h->router_log_thr, h->router_reach, r.dev.la, r.dev.lb,
                     r.dev.lc, r.dev.ld,
                     l32, l64, cnt, stride, ls);
             else
-                route_units_kernel<<<rgrid, 128, 0, st>>>(h->units.p, r.unit0, r.n_units, h->launches.p,
+                route_units_kernel<<<rgrid, 128, 0, cs>>>(h->units.p, r.unit0, r.n_units, h->launches.p,
                                                           h->pairs.p, h->Dsh.p, nsh, h->plan.tau, route, l32,
                                                           l64, cnt, stride, ls);
             KArgs a32 = a, a64 = a;
@@ -1905,8 +1930,8 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
                 a32.Jp = h->Jp32.p;
                 a32.Kp = h->Kp32.p;
             }
-            CUDA_OK(h, launch_run32(r, st, a32));
-            CUDA_OK(h, launch_run(r, st, a64));
+            CUDA_OK(h, launch_run32(r, cs, a32));
+            CUDA_OK(h, launch_run(r, cs, a64));
             launches += 3;
             if (check) {  // the sample of the FP32 queue, in FP32 and in FP64
                 KArgs s32 = a32, s64 = a64;
@@ -1917,16 +1942,17 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
                 s64.Jp = h->EJ64.p;
                 s64.Kp = h->EK64.p;
                 s32.computed = s64.computed = nullptr;
-                CUDA_OK(h, launch_run32(r, st, s32));
-                CUDA_OK(h, launch_run(r, st, s64));
+                CUDA_OK(h, launch_run32(r, cs, s32));
+                CUDA_OK(h, launch_run(r, cs, s64));
                 launches += 2;
             }
         } else {
-            CUDA_OK(h, launch_run(r, st, a));
+            CUDA_OK(h, launch_run(r, cs, a));
             ++launches;
         }
-        CUDA_OK(h, cudaEventRecordWithFlags(h->cev[ri].second, st, ev_flags));
+        CUDA_OK(h, cudaEventRecordWithFlags(h->cev[ri].second, cs, ev_flags));
     }
+    if (overlap) CUDA_OK(h, h->side.join(st));
     if (scatter) {
         // the bra blocks' partials in unit order, then each launch's scatter
         // in launch order: J' and K' are the same sums in the same order on
@@ -1952,8 +1978,11 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
                                                h->check_est.p);
         zero_if_kernel<<<cgrid, 256, 0, st>>>(h->Jp32.p, h->Kp32.p, nn, h->check_flag.p);
         launches += 3;
-        for (size_t ri = 0; ri < h->runs.size(); ++ri) {
+        if (overlap) CUDA_OK(h, h->side.fork(st));
+        for (size_t rj = 0; rj < h->runs.size(); ++rj) {
+            const size_t ri = h->runs.size() - 1 - rj;
             const ClassRun &r = h->runs[ri];
+            const cudaStream_t cs = overlap ? h->side.s[rj % SideStreams::kN] : st;
             KArgs a{};
             a.C = r.dev;
             a.units = h->units.p + r.unit0;
@@ -1971,9 +2000,10 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
             a.boys_tab = h->boys.p;
             a.unit_list = h->route_list.p + r.unit0;
             a.unit_count = h->route_counts.p + 4 * ri + 3;
-            CUDA_OK(h, launch_run(r, st, a));
+            CUDA_OK(h, launch_run(r, cs, a));
             ++launches;
         }
+        if (overlap) CUDA_OK(h, h->side.join(st));
     }
     h->built = true;
     CUDA_OK(h, cudaEventRecordWithFlags(h->ev1, st, ev_flags));
@@ -2002,6 +2032,8 @@ int fjb_fock_build_graph(fjb_handle *h, const double *D_dev, double *J_dev, doub
                       h->g_thr == threshold;
     if (!same) {
         h->drop_graph();
+        bool overlap = false;  // the side streams are made before the capture
+        CUDA_OK(h, use_side_streams(h->side, h->n_units, false, &overlap));
         if (!h->cap_stream) CUDA_OK(h, cudaStreamCreateWithFlags(&h->cap_stream, cudaStreamNonBlocking));
         CUDA_OK(h, cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal));
         const int rc = fjb_fock_build(h, D_dev, J_dev, K_dev, G_dev, precision, threshold, h->cap_stream);
@@ -3209,6 +3241,7 @@ struct fjb_batch {
     size_t max_nn = 0;
     DevBuf<int> route_list, route_counts;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    SideStreams side;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> cev;
     bool ready = false;  // densities set
     std::string err;
@@ -3432,9 +3465,14 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
     const unsigned ev_flags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     BCUDA_OK(b, cudaEventRecordWithFlags(b->ev0, st, ev_flags));
     const fjb_handle *h0 = b->mols[0];
-    for (size_t ri = 0; ri < b->runs.size(); ++ri) {
+    bool overlap = false;
+    BCUDA_OK(b, use_side_streams(b->side, b->n_units, cap == cudaStreamCaptureStatusActive, &overlap));
+    if (overlap) BCUDA_OK(b, b->side.fork(st));
+    for (size_t rj = 0; rj < b->runs.size(); ++rj) {
+        const size_t ri = b->runs.size() - 1 - rj;
         const ClassRun &r = b->runs[ri];
-        BCUDA_OK(b, cudaEventRecordWithFlags(b->cev[ri].first, st, ev_flags));
+        const cudaStream_t cs = overlap ? b->side.s[rj % SideStreams::kN] : st;
+        BCUDA_OK(b, cudaEventRecordWithFlags(b->cev[ri].first, cs, ev_flags));
         KArgs a{};
         a.C = r.dev;
         a.units = b->units.p + r.unit0;
@@ -3455,13 +3493,13 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
             const int rgrid = std::max(1, std::min((r.n_units + 3) / 4, 16 * sm_count()));
             // the first molecule's learned router routes the whole batch
             if (h0->router_on && r.dev.la + r.dev.lb + r.dev.lc + r.dev.ld >= h0->router_min_l)
-                route_units_mlp_kernel<<<rgrid, 128, 0, st>>>(
+                route_units_mlp_kernel<<<rgrid, 128, 0, cs>>>(
                     b->units.p, r.unit0, r.n_units, b->launches.p, b->pairs.p, b->prims.p, nullptr, 0, b->tau,
                     route, h0->router_p.p, h0->router_log_thr, h0->router_reach, r.dev.la, r.dev.lb, r.dev.lc,
                     r.dev.ld, l32, l64,
                     cnt, 0, nullptr, b->ctx.p, b->launch_mol.p);
             else
-                route_units_kernel<<<rgrid, 128, 0, st>>>(b->units.p, r.unit0, r.n_units, b->launches.p,
+                route_units_kernel<<<rgrid, 128, 0, cs>>>(b->units.p, r.unit0, r.n_units, b->launches.p,
                                                           b->pairs.p, nullptr, 0, b->tau, route, l32, l64, cnt, 0,
                                                           nullptr, b->ctx.p, b->launch_mol.p);
             KArgs a32 = a, a64 = a;
@@ -3469,12 +3507,12 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
             a32.unit_count = cnt;
             a64.unit_list = l64;
             a64.unit_count = cnt + 1;
-            BCUDA_OK(b, launch_run32(r, st, a32));
-            BCUDA_OK(b, launch_run(r, st, a64));
+            BCUDA_OK(b, launch_run32(r, cs, a32));
+            BCUDA_OK(b, launch_run(r, cs, a64));
         } else {
-            BCUDA_OK(b, launch_run(r, st, a));
+            BCUDA_OK(b, launch_run(r, cs, a));
         }
-        BCUDA_OK(b, cudaEventRecordWithFlags(b->cev[ri].second, st, ev_flags));
+        BCUDA_OK(b, cudaEventRecordWithFlags(b->cev[ri].second, cs, ev_flags));
     }
     BCUDA_OK(b, cudaEventRecordWithFlags(b->ev1, st, ev_flags));
     const unsigned cx = (unsigned)std::min<size_t>((b->max_nn + 255) / 256, 1024);
@@ -3494,6 +3532,7 @@ int fjb_batch_stats(const fjb_batch *bc, double *ms, int64_t *n_classes, int64_t
         BCUDA_OK(b, cudaEventElapsedTime(&f, b->ev0, b->ev1));
         *ms = f;
     }
+    if (overlap) BCUDA_OK(b, b->side.join(st));
     return FJB_OK;
 }
 

@@ -62,6 +62,8 @@ cudaError_t rys_launch(int la, int lb, int lc, int ld, bool fp32, int grid, cuda
 
 namespace rys {
 
+constexpr int kItemsPerCta = 6;  // below this many items a CTA, units are cut into slices
+
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 __host__ __device__ constexpr int nrange(int lo, int hi) {
     int n = 0;
@@ -340,8 +342,14 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
     const int G = L.group, P = L.chunk;
     const int KSTR = S::template kstride<R>(P);
     const int n_todo = A.unit_list ? *A.unit_count : A.n_units;
+    // a queue short for the grid: each unit's groups over several CTAs
+    const int max_slices = (kKetChunk + G - 1) / G;
+    int ns = n_todo > 0 ? rys::kItemsPerCta * (int)gridDim.x / n_todo : 1;
+    ns = ns < 1 ? 1 : (ns > max_slices ? max_slices : ns);
+    const int n_items = n_todo * ns;
 
-    for (int ui = blockIdx.x; ui < n_todo; ui += gridDim.x) {
+    for (int item_i = blockIdx.x; item_i < n_items; item_i += gridDim.x) {
+        const int ui = item_i / ns, slice = item_i - ui * ns;
         const int u = A.unit_list ? A.unit_list[ui] : ui;
         const Unit U = A.units[u];
         const LaunchRec LR = A.launches[U.launch];
@@ -380,7 +388,7 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
         const int K = kab * kcd;
         const double bra_deg = bra.a == bra.b ? 0.5 : 1.0;
 
-        for (int g0 = 0; g0 < n_list; g0 += G) {
+        for (int g0 = slice * G; g0 < n_list; g0 += G * ns) {
             const int ng = min(G, n_list - g0);
             // -- the group's kets: primitive pairs, HRR coefficients, densities
             for (int i = tid; i < ng * kcd * kPrimWords; i += NT) {
@@ -621,8 +629,8 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
             __syncthreads();
         }
         for (int i = tid; i < NAB; i += NT)
-            if (Jab[i] != 0.0) atomicAdd(M.Jp + (size_t)(oa + i / NB) * n_ao + ob + i % NB, Jab[i]);
-        if (A.computed && tid == 0 && n_list) atomicAdd(A.computed + U.launch, (unsigned long long)n_list);
+            if (Jab[i] != 0.0) red_add(M.Jp + (size_t)(oa + i / NB) * n_ao + ob + i % NB, Jab[i]);
+        if (A.computed && tid == 0 && slice == 0 && n_list) atomicAdd(A.computed + U.launch, (unsigned long long)n_list);
         __syncthreads();
     }
 }
