@@ -48,15 +48,12 @@
 #include <utility>
 
 #include "fock_compiled.cuh"
+#include "hermite_r.cuh"
+#include "jrys.h"
 
 namespace fjb {
 
 namespace {
-
-constexpr int kJMaxL = 2 * kMaxL;  // L of one record
-constexpr int kNHMax = (kJMaxL + 1) * (kJMaxL + 2) * (kJMaxL + 3) / 6;  // 84
-
-__host__ __device__ constexpr int nh(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }
 
 // cartesians(l) components for l <= 3, at offset l(l+1)(l+2)/6.
 __constant__ int8_t kCart[20][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2, 0, 0}, {1, 1, 0}, {1, 0, 1},
@@ -66,14 +63,6 @@ __constant__ int8_t kCart[20][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, 
 // Hermite indices (t, u, v) of hermite_order(2 * kJMaxL), for R tables.
 constexpr int kNRMax = nh(2 * kJMaxL);  // 455
 __constant__ int8_t kHermR[kNRMax][3];
-
-struct JRec {
-    double P[3], PA[3], PB[3];
-    double zeta, pre, G;  // pre = c_a c_b (pi/zeta)^{3/2} exp(-alpha beta/zeta |AB|^2)
-    int32_t la, lb, ao_a, ao_b;
-    int32_t L, pair, dq_off, pad;
-};
-static_assert(sizeof(JRec) == 128, "JRec is 128 bytes");
 
 constexpr int kETab = 4 * 4 * (kJMaxL + 1);  // E[i][j][t], i, j <= 3, t <= 6
 
@@ -141,89 +130,6 @@ __global__ void j_dq_kernel(const JRec *__restrict__ recs, int n, const double *
     }
 }
 
-__device__ __forceinline__ int h_index(int t, int u, int v) {
-    const int n = t + u + v;
-    return (n == 0 ? 0 : nh(n - 1)) + (n - t) * (n - t + 1) / 2 + (n - t - u);
-}
-
-// hermite_order index -> (t, u, v), constexpr, for the unrolled kernels.
-__host__ __device__ constexpr int hc_total(int idx) {
-    int n = 0;
-    while (nh(n) <= idx) ++n;
-    return n;
-}
-__host__ __device__ constexpr int hc_t(int idx) {
-    const int n = hc_total(idx);
-    int r = idx - (n == 0 ? 0 : nh(n - 1)), t = n;
-    while (r >= n - t + 1) {
-        r -= n - t + 1;
-        --t;
-    }
-    return t;
-}
-__host__ __device__ constexpr int hc_u(int idx) {
-    const int n = hc_total(idx);
-    int r = idx - (n == 0 ? 0 : nh(n - 1)), t = n;
-    while (r >= n - t + 1) {
-        r -= n - t + 1;
-        --t;
-    }
-    return n - t - r;
-}
-__host__ __device__ constexpr int hc_v(int idx) { return hc_total(idx) - hc_t(idx) - hc_u(idx); }
-__host__ __device__ constexpr int hc_idx(int t, int u, int v) {
-    const int n = t + u + v;
-    return (n == 0 ? 0 : nh(n - 1)) + (n - t) * (n - t + 1) / 2 + (n - t - u);
-}
-
-// Compile-time walks of the small classes: every index below is a template
-// constant (fold expressions over integer sequences), so R, the signed D_q
-// and the J_p partials stay in registers.
-// One entry I of the R recursion: [r]^(m) = PQ_d [r-1_d]^(m+1) + (r_d - 1)
-// [r-2_d]^(m+1), d the first nonzero axis.
-template <int I, typename T>
-__device__ __forceinline__ void r_entry(T *R, T X, T Y, T Z) {
-    constexpr int t = hc_t(I), u = hc_u(I), v = hc_v(I);
-    if constexpr (t > 0) {
-        T x = X * R[hc_idx(t - 1, u, v)];
-        if constexpr (t >= 2) x += (T)(t - 1) * R[hc_idx(t - 2, u, v)];
-        R[I] = x;
-    } else if constexpr (u > 0) {
-        T x = Y * R[hc_idx(0, u - 1, v)];
-        if constexpr (u >= 2) x += (T)(u - 1) * R[hc_idx(0, u - 2, v)];
-        R[I] = x;
-    } else {
-        T x = Z * R[hc_idx(0, 0, v - 1)];
-        if constexpr (v >= 2) x += (T)(v - 1) * R[hc_idx(0, 0, v - 2)];
-        R[I] = x;
-    }
-}
-template <int I0, typename T, int... K>
-__device__ __forceinline__ void r_entries(T *R, T X, T Y, T Z, std::integer_sequence<int, K...>) {
-    (r_entry<I0 + K, T>(R, X, Y, Z), ...);
-}
-// Totals S, S-1, .. 1 of one level (descending: each reads the level above
-// at totals S-1 and S-2 before they are rewritten).
-template <int S, typename T>
-struct RTotals {
-    static __device__ __forceinline__ void run(T *R, T X, T Y, T Z) {
-        if constexpr (S >= 1) {
-            r_entries<nh(S - 1), T>(R, X, Y, Z, std::make_integer_sequence<int, nh(S) - nh(S - 1)>{});
-            RTotals<S - 1, T>::run(R, X, Y, Z);
-        }
-    }
-};
-// Levels M, M-1, .. 0 of R_{tuv} at total order L.
-template <int L, int M, typename T>
-struct RLevels {
-    static __device__ __forceinline__ void run(T *R, const T *f, T X, T Y, T Z) {
-        if constexpr (M >= 0) {
-            RTotals<L - M, T>::run(R, X, Y, Z);
-            R[0] = f[M];
-            RLevels<L, M - 1, T>::run(R, f, X, Y, Z);
-        }
-    }
-};
 // d[q] = (-1)^|q| D_q.
 template <typename T, int... Q>
 __device__ __forceinline__ void signed_dq(T *d, const double *dq, std::integer_sequence<int, Q...>) {
@@ -240,10 +146,7 @@ __device__ __forceinline__ void contract(T *jp, const T *R, const T *d, std::int
     ((jp[PQIndex<NQ, I>::pi] += R[PQIndex<NQ, I>::r] * d[PQIndex<NQ, I>::qi]), ...);
 }
 
-// The classes with lp + lq <= kSmallL: the same walk as j_pq_kernel with
-// every index a compile-time constant.
-constexpr int kSmallL = 6;
-
+// The classes with lp + lq <= kJSmallL: every index a compile-time constant.
 // thr32 > 0: a chunk of kets whose first (largest) bound I_bra key is below
 // it runs R, D_q and the contraction in FP32 (T, the Boys values and the
 // J_p sums stay FP64): the FP32 E/R tier.  The kets are sorted by key, so
@@ -324,147 +227,6 @@ __global__ void __launch_bounds__(128) j_pq_small_kernel(const JRec *__restrict_
     }
 }
 
-// One bra-ket record pair of the table-indexed walk in T (float: the FP32
-// E/R tier): R from the FP64 Boys values, then jp[p] += R_{p+q} (-1)^|q| D_q
-// summed in T over the ket and added to the FP64 partials.
-template <int L, typename T>
-__device__ __forceinline__ void pq_lane_general(const JRec &B, double4 KP, const double *dq, int lp, int lq,
-                                                const double *boys_tab, double *jp) {
-    constexpr int NR = nh(L);
-    constexpr double kTwoOverSqrtPi = 1.1283791670955126;
-    const int NP = nh(lp), NQ = nh(lq);
-    const double p = B.zeta, q = KP.w;
-    const double rho = p * q / (p + q);
-    const double Xd = B.P[0] - KP.x, Yd = B.P[1] - KP.y, Zd = B.P[2] - KP.z;
-    const double Tt = rho * (Xd * Xd + Yd * Yd + Zd * Zd);
-    double F[L + 1];
-    boys_t<L>(Tt, F, boys_tab);
-    const double pref = kTwoOverSqrtPi * sqrt(rho), m2r = -2.0 * rho;
-    T f[L + 1];
-    double pw = pref;
-#pragma unroll
-    for (int m = 0; m <= L; ++m) {
-        f[m] = (T)(pw * F[m]);
-        pw *= m2r;
-    }
-    const T X = (T)Xd, Y = (T)Yd, Z = (T)Zd;
-    T R[NR];
-    R[0] = f[L];
-    for (int m = L - 1; m >= 0; --m) {
-        for (int s = L - m; s >= 1; --s) {
-            for (int i = nh(s - 1); i < nh(s); ++i) {
-                const int t = kHermR[i][0], u = kHermR[i][1], v = kHermR[i][2];
-                T x;
-                if (t > 0) {
-                    x = X * R[h_index(t - 1, u, v)];
-                    if (t >= 2) x += (T)(t - 1) * R[h_index(t - 2, u, v)];
-                } else if (u > 0) {
-                    x = Y * R[h_index(0, u - 1, v)];
-                    if (u >= 2) x += (T)(u - 1) * R[h_index(0, u - 2, v)];
-                } else {
-                    x = Z * R[h_index(0, 0, v - 1)];
-                    if (v >= 2) x += (T)(v - 1) * R[h_index(0, 0, v - 2)];
-                }
-                R[i] = x;
-            }
-        }
-        R[0] = f[m];
-    }
-    for (int pi = 0; pi < NP; ++pi) {
-        T acc = (T)0;
-        for (int qi = 0; qi < NQ; ++qi) {
-            const int tq = kHermR[qi][0], uq = kHermR[qi][1], vq = kHermR[qi][2];
-            const T d = (T)((((tq + uq + vq) & 1) ? -1.0 : 1.0) * __ldg(dq + qi));
-            acc += R[h_index(kHermR[pi][0] + tq, kHermR[pi][1] + uq, kHermR[pi][2] + vq)] * d;
-        }
-        jp[pi] += (double)acc;
-    }
-}
-
-// One (bra L, ket L) class at total order L = lp + lq (runtime lp, lq).
-template <int L>
-__global__ void __launch_bounds__(128) j_pq_kernel(const JRec *__restrict__ recs, int lp, int lq, int bra0, int nbra,
-                                                   int ket0, int nket, const double4 *__restrict__ kst, const int *__restrict__ kdq,
-                                                   const double *__restrict__ skey, const double *__restrict__ Dq,
-                                                   double *__restrict__ Jp, double tau, double thr32,
-                                                   const double *__restrict__ boys_tab) {
-    constexpr int NR = nh(L), NPMAX = nh(L < kJMaxL ? L : kJMaxL);
-    constexpr double kTwoOverSqrtPi = 1.1283791670955126;
-    const int NP = nh(lp), NQ = nh(lq);
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int bi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); bi < nbra; bi += nw) {
-        const JRec B = recs[bra0 + bi];
-        double jp[NPMAX];
-        for (int p = 0; p < NP; ++p) jp[p] = 0.0;
-        for (int k0 = 0; k0 < nket; k0 += 32) {
-            const int k = k0 + lane;
-            const bool on = k < nket && !(B.G * skey[ket0 + k] < tau);
-            const bool f32 = thr32 > 0.0 && B.G * skey[ket0 + k0] < thr32;  // uniform over the warp
-            if (on && f32) {
-                pq_lane_general<L, float>(B, kst[ket0 + k], Dq + kdq[ket0 + k], lp, lq, boys_tab, jp);
-            } else if (on) {
-                const double4 KP = kst[ket0 + k];  // (P, eta) of the k-th ket in key order
-                const int kdo = kdq[ket0 + k];
-                const double p = B.zeta, q = KP.w;
-                const double rho = p * q / (p + q);
-                const double X = B.P[0] - KP.x, Y = B.P[1] - KP.y, Z = B.P[2] - KP.z;
-                const double T = rho * (X * X + Y * Y + Z * Z);
-                double F[L + 1];
-                boys_t<L>(T, F, boys_tab);
-                const double pref = kTwoOverSqrtPi * sqrt(rho), m2r = -2.0 * rho;
-                double f[L + 1];
-                double pw = pref;
-#pragma unroll
-                for (int m = 0; m <= L; ++m) {
-                    f[m] = pw * F[m];
-                    pw *= m2r;
-                }
-                // R_{tuv}: level m = L holds [0]^(L); each lower level
-                // rewrites totals L-m .. 1 from the level above (read before
-                // they are overwritten: totals descend), then [0]^(m).
-                double R[NR];
-                R[0] = f[L];
-                for (int m = L - 1; m >= 0; --m) {
-                    for (int s = L - m; s >= 1; --s) {
-                        for (int i = nh(s - 1); i < nh(s); ++i) {
-                            const int t = kHermR[i][0], u = kHermR[i][1], v = kHermR[i][2];
-                            double x;
-                            if (t > 0) {
-                                x = X * R[h_index(t - 1, u, v)];
-                                if (t >= 2) x += (double)(t - 1) * R[h_index(t - 2, u, v)];
-                            } else if (u > 0) {
-                                x = Y * R[h_index(0, u - 1, v)];
-                                if (u >= 2) x += (double)(u - 1) * R[h_index(0, u - 2, v)];
-                            } else {
-                                x = Z * R[h_index(0, 0, v - 1)];
-                                if (v >= 2) x += (double)(v - 1) * R[h_index(0, 0, v - 2)];
-                            }
-                            R[i] = x;
-                        }
-                    }
-                    R[0] = f[m];
-                }
-                const double *dq = Dq + kdo;
-                for (int qi = 0; qi < NQ; ++qi) {
-                    const int tq = kHermR[qi][0], uq = kHermR[qi][1], vq = kHermR[qi][2];
-                    const double d = (((tq + uq + vq) & 1) ? -1.0 : 1.0) * __ldg(dq + qi);
-                    for (int pi = 0; pi < NP; ++pi)
-                        jp[pi] += R[h_index(kHermR[pi][0] + tq, kHermR[pi][1] + uq, kHermR[pi][2] + vq)] * d;
-                }
-            }
-            const unsigned bal = __ballot_sync(0xffffffffu, on);
-            if (__popc(bal) < min(32, nket - k0)) break;  // the first ket under tau is in this chunk
-        }
-        for (int pi = 0; pi < NP; ++pi) {
-            double v = jp[pi];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) Jp[B.dq_off + pi] += v;
-        }
-    }
-}
-
 // The kets of every L in key order as a contiguous stream: (P, eta) of the
 // k-th sorted ket, and its D_q copied into the D_q slot of position k (a
 // group's slots have one stride, so position k's slot is record k's), so the
@@ -521,23 +283,6 @@ __global__ void j_jab_kernel(const JRec *__restrict__ recs, const int *__restric
     }
 }
 
-using PqLaunch = void (*)(int grid, cudaStream_t st, const JRec *, int, int, int, int, int, int, const double4 *,
-                          const int *, const double *, const double *, double *, double, double, const double *);
-
-template <int L>
-void pq_launch(int grid, cudaStream_t st, const JRec *recs, int lp, int lq, int bra0, int nbra, int ket0, int nket,
-               const double4 *kst, const int *kdq, const double *skey, const double *Dq, double *Jp, double tau,
-               double thr32, const double *boys) {
-    j_pq_kernel<L><<<grid, 128, 0, st>>>(recs, lp, lq, bra0, nbra, ket0, nket, kst, kdq, skey, Dq, Jp, tau, thr32,
-                                         boys);
-}
-
-template <int... L>
-constexpr std::array<PqLaunch, sizeof...(L)> pq_table(std::integer_sequence<int, L...>) {
-    return {&pq_launch<L>...};
-}
-const auto kPqTable = pq_table(std::make_integer_sequence<int, 2 * kJMaxL + 1>{});
-
 using PqSmallLaunch = void (*)(int grid, cudaStream_t st, const JRec *, int, int, int, int, const double4 *,
                                const int *, const double *, const double *, double *, double, double,
                                const double *);
@@ -546,7 +291,7 @@ template <int LP, int LQ>
 void pq_small_launch(int grid, cudaStream_t st, const JRec *recs, int bra0, int nbra, int ket0, int nket,
                      const double4 *kst, const int *kdq, const double *skey, const double *Dq, double *Jp, double tau,
                      double thr32, const double *boys) {
-    if constexpr (LP + LQ <= kSmallL)
+    if constexpr (LP + LQ <= kJSmallL)
         j_pq_small_kernel<LP, LQ><<<grid, 128, 0, st>>>(recs, bra0, nbra, ket0, nket, kst, kdq, skey, Dq, Jp,
                                                         tau, thr32, boys);
 }
@@ -708,7 +453,8 @@ JEngine *jengine_create(const HostBasis &basis, int device, std::string *err) {
 void jengine_destroy(JEngine *e) { delete e; }
 
 int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, double thr32, const double *boys_tab,
-                  cudaStream_t st, std::string *err, int *launches) {
+                  const double *rys_tab, const float *rys_tab32, SideStreams *side, cudaStream_t st, std::string *err,
+                  int *launches) {
     int nl = 0;
     auto check = [&](cudaError_t c, const char *what) {
         if (c == cudaSuccess) return true;
@@ -734,23 +480,30 @@ int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, do
     ++nl;
     if (!check(cudaGetLastError(), "j_gather_kernel")) return -2;
     if (!check(cudaMemsetAsync(e->Jp.p, 0, e->Jp.n * sizeof(double), st), "memset")) return -2;
-    for (int lp = 0; lp <= kJMaxL; ++lp) {
+    // a bra order's classes add into the same J_p, in turn on one stream; the
+    // bra orders run side by side
+    if (side && !check(side->fork(st), "fork")) return -2;
+    for (int lp = kJMaxL; lp >= 0; --lp) {
+        const cudaStream_t cs = side ? side->s[lp] : st;
         const int b0 = e->L_off[lp], nb = e->L_off[lp + 1] - b0;
         if (nb == 0) continue;
         const int grid = std::max(1, std::min((nb + 3) / 4, sms * 8));
         for (int lq = 0; lq <= kJMaxL; ++lq) {
             const int k0 = e->L_off[lq], nk = e->L_off[lq + 1] - k0;
             if (nk == 0) continue;
-            if (lp + lq <= kSmallL)
-                kPqSmall[lp][lq](grid, st, e->recs.p, b0, nb, k0, nk, e->kst.p, e->kdq.p, e->skey.p, e->Dqs.p, e->Jp.p, tau,
+            if (lp + lq <= kJSmallL)
+                kPqSmall[lp][lq](grid, cs, e->recs.p, b0, nb, k0, nk, e->kst.p, e->kdq.p, e->skey.p, e->Dqs.p, e->Jp.p, tau,
                                  thr32, boys_tab);
             else
-                kPqTable[lp + lq](grid, st, e->recs.p, lp, lq, b0, nb, k0, nk, e->kst.p, e->kdq.p, e->skey.p, e->Dqs.p,
-                                  e->Jp.p, tau, thr32, boys_tab);
+                if (!check(j_rys_launch(lp, lq, cs, JRysArgs{e->recs.p, b0, nb, k0, nk, e->kst.p, e->kdq.p, e->skey.p, e->Dqs.p,
+                                                  e->Jp.p, tau, thr32, rys_tab, rys_tab32}),
+                           "j_rys_kernel"))
+                    return -2;
             ++nl;
-            if (!check(cudaGetLastError(), "j_pq_kernel")) return -2;
+            if (!check(cudaGetLastError(), "j_pq_small_kernel")) return -2;
         }
     }
+    if (side && !check(side->join(st), "join")) return -2;
     const int pair_grid = std::max(1, std::min((e->n_pairs + 3) / 4, sms * 16));
     j_jab_kernel<<<pair_grid, 128, 0, st>>>(e->recs.p, e->pair_rec0.p, e->pair_nrec.p, e->n_pairs, e->Jp.p, J_dev,
                                             e->n_ao);
