@@ -906,10 +906,10 @@ struct ClassRun {
     bool rys64 = false, rys32 = false;
     RysDev ry64{}, ry32{};
     int grid_r64 = 0, grid_r32 = 0;
-    const double *rys_tab = nullptr;
     // the warp-autonomous Rys kernel (rys_warp.cuh), when it takes the class
     bool warp64 = false, warp32 = false;
     int grid_w64 = 0, grid_w32 = 0;
+    const double *rys_tab = nullptr;
     const float *rys_tab32 = nullptr;
     ClassDev dev32;  // the FP32 interpreter's layout (routed builds of classes without has32)
     int unit0 = 0, n_units = 0;
@@ -957,12 +957,12 @@ int run_grid(const ClassRun &r);
 // The FP64 path of a class run: its register kernel, else the Rys kernel,
 // else the interpreter (which alone serves the atomics-free build's slots).
 cudaError_t launch_run(const ClassRun &r, cudaStream_t st, const KArgs &a) {
-    if (r.rys64 && !a.W) {
     if (r.warp64 && !a.W) {
         KArgs ar = a;
         ar.rys_tab = r.rys_tab;
         return rys_warp_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, false, r.grid_w64, st, ar);
     }
+    if (r.rys64 && !a.W) {
         KArgs ar = a;
         ar.Y = r.ry64;
         ar.rys_tab = r.rys_tab;
@@ -976,12 +976,12 @@ cudaError_t launch_run(const ClassRun &r, cudaStream_t st, const KArgs &a) {
 // The FP32 kernel of a class run (routed builds): its register kernel, else
 // the Rys kernel in FP32, else the interpreter in FP32 with its own layout.
 cudaError_t launch_run32(const ClassRun &r, cudaStream_t st, const KArgs &a) {
-    if (r.has32) return launch_compiled(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid32, st, a);
     if (r.warp32 && !a.W) {
         KArgs ar = a;
         ar.rys_tab32 = r.rys_tab32;
         return rys_warp_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid_w32, st, ar);
     }
+    if (r.has32) return launch_compiled(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid32, st, a);
     if (r.rys32 && !a.W) {
         KArgs ar = a;
         ar.Y = r.ry32;
@@ -1435,6 +1435,18 @@ void choose_rys(int mode, ClassRun &r) {
     };
     if (r.rys64) r.grid_r64 = rgrid(false, r.ry64);
     if (r.rys32) r.grid_r32 = rgrid(true, r.ry32);
+    const auto wgrid = [&](bool fp32) {
+        const int64_t most = (int64_t)r.n_units * kKetChunk;  // a unit makes at most one item a ket
+        const int per_sm = std::max(1, rys_warp_blocks_per_sm(la, lb, lc, ld, fp32));
+        return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
+    };
+    const auto wtake = [&](bool fp32) {
+        return mode >= 1 && rys_warp_available(la, lb, lc, ld) && (mode == 2 || rys_warp_preferred(la, lb, lc, ld, fp32));
+    };
+    r.warp64 = wtake(false);
+    r.warp32 = wtake(true);
+    if (r.warp64) r.grid_w64 = wgrid(false);
+    if (r.warp32) r.grid_w32 = wgrid(true);
 }
 
 // The Rys rule's device tables, FP64 and FP32, built once per process
@@ -1453,18 +1465,6 @@ const RysTables &rys_tables_cached() {
 
 int finish_create(std::unique_ptr<fjb_handle> &h, fjb_handle **out) {
     const int device = h->device;
-    const auto wgrid = [&](bool fp32) {
-        const int64_t most = (int64_t)r.n_units * kKetChunk;  // a unit makes at most one item a ket
-        const int per_sm = std::max(1, rys_warp_blocks_per_sm(la, lb, lc, ld, fp32));
-        return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
-    };
-    const auto wtake = [&](bool fp32) {
-        return mode >= 1 && rys_warp_available(la, lb, lc, ld) && (mode == 2 || rys_warp_preferred(la, lb, lc, ld, fp32));
-    };
-    r.warp64 = wtake(false);
-    r.warp32 = wtake(true);
-    if (r.warp64) r.grid_w64 = wgrid(false);
-    if (r.warp32) r.grid_w32 = wgrid(true);
     if (device < 0) {  // host-only handle: plans and exports, no builds
         *out = h.release();
         return FJB_OK;
@@ -3228,6 +3228,7 @@ extern "C" int fjb_fock_build_noalloc(fjb_handle *h, const double *D_dev, double
 
 struct fjb_batch {
     int device = 0;
+    SideStreams side;
     double tau = 0.0;
     std::vector<fjb_handle *> mols;
     DevBuf<PairRec> pairs;
@@ -3246,7 +3247,6 @@ struct fjb_batch {
     size_t max_nn = 0;
     DevBuf<int> route_list, route_counts;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    SideStreams side;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> cev;
     bool ready = false;  // densities set
     std::string err;
@@ -3519,6 +3519,7 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
         }
         BCUDA_OK(b, cudaEventRecordWithFlags(b->cev[ri].second, cs, ev_flags));
     }
+    if (overlap) BCUDA_OK(b, b->side.join(st));
     BCUDA_OK(b, cudaEventRecordWithFlags(b->ev1, st, ev_flags));
     const unsigned cx = (unsigned)std::min<size_t>((b->max_nn + 255) / 256, 1024);
     batch_close_kernel<<<dim3(cx, nm), 256, 0, st>>>(b->bm.p);
@@ -3537,7 +3538,6 @@ int fjb_batch_stats(const fjb_batch *bc, double *ms, int64_t *n_classes, int64_t
         BCUDA_OK(b, cudaEventElapsedTime(&f, b->ev0, b->ev1));
         *ms = f;
     }
-    if (overlap) BCUDA_OK(b, b->side.join(st));
     return FJB_OK;
 }
 
