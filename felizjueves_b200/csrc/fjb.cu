@@ -2796,7 +2796,15 @@ int fjb_df_eri3(fjb_handle *h, int aux_shell0, int aux_shell1, double tau, doubl
     }
     CUDA_OK(h, cudaMemsetAsync(out_dev, 0, (size_t)n_ao * n_ao * nb * sizeof(double), st));
     const int sms = sm_count();
-    for (const Launch &L : launches) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CUDA_OK(h, cudaStreamIsCapturing(st, &cap));
+    bool overlap = false;  // the classes write disjoint blocks: side by side
+    CUDA_OK(h, use_side_streams(h->side, 0, cap == cudaStreamCaptureStatusActive, &overlap));
+    std::reverse(launches.begin(), launches.end());  // the largest classes first
+    if (overlap) CUDA_OK(h, h->side.fork(st));
+    for (size_t li = 0; li < launches.size(); ++li) {
+        const Launch &L = launches[li];
+        const cudaStream_t cs = overlap ? h->side.s[li % SideStreams::kN] : st;
         auto key = std::make_tuple(L.la, L.lb, L.lp);
         auto it = h->e3_dev.find(key);
         if (it == h->e3_dev.end() || it->second.kab < L.max_kab || it->second.kcd < L.max_kcd) {
@@ -2821,9 +2829,10 @@ int fjb_df_eri3(fjb_handle *h, int aux_shell0, int aux_shell1, double tau, doubl
         a.rys_tab = h->rys.p;
         const int per_sm = std::max(1, eri3_blocks_per_sm(L.la, L.lb, L.lp, a.Y));
         const int grid = (int)std::min<size_t>(L.n, (size_t)per_sm * sms);
-        CUDA_OK(h, eri3_launch(L.la, L.lb, L.lp, grid, st, a));
+        CUDA_OK(h, eri3_launch(L.la, L.lb, L.lp, grid, cs, a));
         if (n_launches) ++*n_launches;
     }
+    if (overlap) CUDA_OK(h, h->side.join(st));
     return FJB_OK;
 }
 
