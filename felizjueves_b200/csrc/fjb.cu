@@ -2909,8 +2909,12 @@ int fjb_one_electron(fjb_handle *h, const double *charges, const double *coords,
         if (!h->onee) return fail(h, FJB_E_CUDA, err);
     }
     int nl = 0;
-    if (onee_build(h->onee, charges, coords, n_nuc, S_dev, T_dev, V_dev, H_dev, h->boys.p, (cudaStream_t)stream,
-                   &err, &nl))
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CUDA_OK(h, cudaStreamIsCapturing((cudaStream_t)stream, &cap));
+    bool overlap = false;
+    CUDA_OK(h, use_side_streams(h->side, 0, cap == cudaStreamCaptureStatusActive, &overlap));
+    if (onee_build(h->onee, charges, coords, n_nuc, S_dev, T_dev, V_dev, H_dev, h->boys.p,
+                   overlap ? &h->side : nullptr, (cudaStream_t)stream, &err, &nl))
         return fail(h, FJB_E_CUDA, err);
     return FJB_OK;
 }

@@ -9,10 +9,15 @@
 //   T_ab += c_a c_b (pi/p)^{3/2} (K_x S_y S_z + S_x K_y S_z + S_x S_y K_z),
 //           K_ij = -2 b^2 S_{i,j+2} + b (2j+1) S_ij - j(j-1)/2 S_{i,j-2}
 //                                                             (kinetic.py:61-111)
-//   V_ab += -Z_C c_a c_b (2 pi / p) sum_tuv E^x_t E^y_u E^z_v R_tuv(p, P - C)
-//           per nucleus, R from (-2p)^n F_n(p |PC|^2) by
+//   V_ab += c_a c_b (2 pi / p) sum_tuv E^x_t E^y_u E^z_v Q_tuv,
+//           Q_tuv = sum_C -Z_C R_tuv(p, P - C), R from (-2p)^n F_n(p |PC|^2) by
 //           R^n_{t+1,u,v} = X_PC R^{n+1}_{tuv} + t R^{n+1}_{t-1,u,v} (and u, v)
 //                                                             (potential.py:1-60)
+// The nuclei are summed in the Hermite basis: R is linear in the charges, so
+// the block's transform -- 100 components of up to 64 terms for (ff) -- runs
+// once per primitive pair, where it ran once per nucleus, and R and Q stay in
+// registers (hermite_r.cuh).  The classes run side by side (side_streams.h):
+// each is a few hundred warps long on its own.
 // Every index is a template constant once the loops unroll, so the tables
 // live in registers (the largest classes spill).  The block is written to
 // (A, B) and mirrored to (B, A); a diagonal pair writes its upper triangle
@@ -28,6 +33,7 @@
 #include <vector>
 
 #include "fock_compiled.cuh"
+#include "hermite_r.cuh"
 
 namespace fjb {
 
@@ -78,8 +84,10 @@ __host__ __device__ constexpr int cart_of(int l, int idx, int d) {
 constexpr int kClasses = (kMaxL + 1) * (kMaxL + 2) / 2;  // (la <= lb) classes
 __host__ __device__ constexpr int cls_index(int la, int lb) { return la * (2 * kMaxL + 3 - la) / 2 + (lb - la); }
 
+constexpr int kOneeThreads = 64;
+
 template <int LA, int LB>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kOneeThreads)
     onee_kernel(const OShell *__restrict__ sh, const double *__restrict__ ex, const double *__restrict__ co,
                 const int2 *__restrict__ pairs, int n, const double4 *__restrict__ nuc, int n_nuc, int n_ao,
                 double *S, double *T, double *V, double *H, const double *__restrict__ boys) {
@@ -165,50 +173,30 @@ __global__ void __launch_bounds__(128)
                     for (int c = 0; c < NB; ++c) st_comp(r, c);
             }
             // nuclear attraction
-            const double pref = ca * cb * 2.0 * kPi * ip;
-            for (int q = 0; q < n_nuc; ++q) {
-                const double4 C = nuc[q];
-                const double pc[3] = {P[0] - C.x, P[1] - C.y, P[2] - C.z};
-                const double x = p * (pc[0] * pc[0] + pc[1] * pc[1] + pc[2] * pc[2]);
-                double F[L + 1];
-                boys_t<L>(x, F, boys);
-                double Rp[L + 1][L + 1][L + 1], Rc[L + 1][L + 1][L + 1];
-                double pws[L + 1];  // (-2p)^m
-                pws[0] = 1.0;
+            if (n_nuc > 0) {
+                const double pref = ca * cb * 2.0 * kPi * ip;
+                constexpr int NH = nh(L);
+                double Q[NH];
 #pragma unroll
-                for (int m = 1; m <= L; ++m) pws[m] = pws[m - 1] * (-2.0 * p);
+                for (int i = 0; i < NH; ++i) Q[i] = 0.0;
+#pragma unroll 1
+                for (int q = 0; q < n_nuc; ++q) {
+                    const double4 C = nuc[q];
+                    const double X = P[0] - C.x, Y = P[1] - C.y, Z = P[2] - C.z;
+                    double F[L + 1];
+                    boys_t<L>(p * (X * X + Y * Y + Z * Z), F, boys);
+                    double pw = -C.w;  // -Z (-2p)^m
 #pragma unroll
-                for (int m = L; m >= 0; --m) {
+                    for (int m = 0; m <= L; ++m) {
+                        F[m] *= pw;
+                        pw *= -2.0 * p;
+                    }
+                    double Rv[NH];
+                    Rv[0] = F[L];
+                    RLevels<L, L - 1, double>::run(Rv, F, X, Y, Z);
 #pragma unroll
-                    for (int sum = 0; sum <= L - m; ++sum)
-#pragma unroll
-                        for (int ti = sum; ti >= 0; --ti)
-#pragma unroll
-                            for (int ui = sum - ti; ui >= 0; --ui) {
-                                const int vi = sum - ti - ui;
-                                double r;
-                                if (sum == 0) {
-                                    r = pws[m] * F[m];
-                                } else if (ti > 0) {
-                                    r = pc[0] * Rp[ti - 1][ui][vi];
-                                    if (ti > 1) r += (double)(ti - 1) * Rp[ti > 1 ? ti - 2 : 0][ui][vi];
-                                } else if (ui > 0) {
-                                    r = pc[1] * Rp[ti][ui - 1][vi];
-                                    if (ui > 1) r += (double)(ui - 1) * Rp[ti][ui > 1 ? ui - 2 : 0][vi];
-                                } else {
-                                    r = pc[2] * Rp[ti][ui][vi - 1];
-                                    if (vi > 1) r += (double)(vi - 1) * Rp[ti][ui][vi > 1 ? vi - 2 : 0];
-                                }
-                                Rc[ti][ui][vi] = r;
-                            }
-#pragma unroll
-                    for (int sum = 0; sum <= L - m; ++sum)
-#pragma unroll
-                        for (int ti = sum; ti >= 0; --ti)
-#pragma unroll
-                            for (int ui = sum - ti; ui >= 0; --ui) Rp[ti][ui][sum - ti - ui] = Rc[ti][ui][sum - ti - ui];
+                    for (int i = 0; i < NH; ++i) Q[i] += Rv[i];
                 }
-                const double w = -C.w * pref;
                 auto v_comp = [&](int r, int c) {
                     const int ax = cart_of(LA, r, 0), ay = cart_of(LA, r, 1), az = cart_of(LA, r, 2);
                     const int bx = cart_of(LB, c, 0), by = cart_of(LB, c, 1), bz = cart_of(LB, c, 2);
@@ -216,9 +204,10 @@ __global__ void __launch_bounds__(128)
                     for (int ti = 0; ti <= ax + bx; ++ti)
                         for (int ui = 0; ui <= ay + by; ++ui) {
                             const double exy = E[0][ax][bx][ti] * E[1][ay][by][ui];
-                            for (int vi = 0; vi <= az + bz; ++vi) acc += exy * E[2][az][bz][vi] * Rp[ti][ui][vi];
+                            for (int vi = 0; vi <= az + bz; ++vi)
+                                acc += exy * E[2][az][bz][vi] * Q[hc_idx(ti, ui, vi)];
                         }
-                    v[r * NB + c] += w * acc;
+                    v[r * NB + c] += pref * acc;
                 };
                 if constexpr (kUnrolled) {
 #pragma unroll
@@ -321,7 +310,8 @@ OneElectron *onee_create(const HostBasis &basis, int device, std::string *err) {
 void onee_destroy(OneElectron *e) { delete e; }
 
 int onee_build(OneElectron *e, const double *charges, const double *coords, int n_nuc, double *S, double *T,
-               double *V, double *H, const double *boys_tab, cudaStream_t st, std::string *err, int *launches) {
+               double *V, double *H, const double *boys_tab, SideStreams *side, cudaStream_t st, std::string *err,
+               int *launches) {
     std::vector<double4> nuc(n_nuc);
     for (int q = 0; q < n_nuc; ++q)
         nuc[q] = make_double4(coords[3 * q], coords[3 * q + 1], coords[3 * q + 2], charges[q]);
@@ -337,14 +327,17 @@ int onee_build(OneElectron *e, const double *charges, const double *coords, int 
         return 1;
     }
     int nl = 0;
-    for (int c = 0; c < kClasses; ++c) {
+    if (side) ce = side->fork(st);
+    for (int c = kClasses - 1; c >= 0 && ce == cudaSuccess; --c) {
         const int n = e->cls_off[c + 1] - e->cls_off[c];
         if (n == 0) continue;
-        kFns[c].fn<<<(n + 127) / 128, 128, 0, st>>>(e->shells.p, e->ex.p, e->co.p, e->pairs.p + e->cls_off[c], n,
+        const cudaStream_t cs = side ? side->s[c % SideStreams::kN] : st;
+        kFns[c].fn<<<(n + kOneeThreads - 1) / kOneeThreads, kOneeThreads, 0, cs>>>(e->shells.p, e->ex.p, e->co.p, e->pairs.p + e->cls_off[c], n,
                                                    e->nuc.p, n_nuc, e->n_ao, S, T, V, H, boys_tab);
         ++nl;
+        ce = cudaGetLastError();
     }
-    ce = cudaGetLastError();
+    if (side && ce == cudaSuccess) ce = side->join(st);
     if (ce != cudaSuccess) {
         *err = std::string("one-electron launch: ") + cudaGetErrorString(ce);
         return 1;

@@ -14,6 +14,7 @@
 #include <string>
 
 #include "plan.h"
+#include "side_streams.h"
 
 namespace fjb {
 
@@ -27,9 +28,9 @@ void onee_destroy(OneElectron *e);
 // S, T, V, H = T + V (n_ao^2, DEVICE, row-major; each may be null and is then
 // not written, every element of the others is written) for nuclei
 // (charges[k], coords[3k..3k+2]) given on the host.  *launches receives the
-// kernel launches issued.
+// kernel launches issued.  side: the streams its classes run on (null: st).
 int onee_build(OneElectron *e, const double *charges, const double *coords, int n_nuc, double *S,
-               double *T, double *V, double *H, const double *boys_tab, cudaStream_t st, std::string *err,
-               int *launches);
+               double *T, double *V, double *H, const double *boys_tab, SideStreams *side, cudaStream_t st,
+               std::string *err, int *launches);
 
 }  // namespace fjb
