@@ -996,6 +996,10 @@ cudaError_t launch_run32(const ClassRun &r, cudaStream_t st, const KArgs &a) {
 
 }  // namespace
 
+// Launches of one class in one build: FP64, FP32, the sample's FP32 and FP64,
+// the re-run; each has a work counter of its own.
+constexpr int kCounters = 8;
+
 // Builds of at most this many work units overlap their class launches.
 constexpr int kOverlapUnits = 1 << 22;
 
@@ -1065,6 +1069,7 @@ struct fjb_handle {
     // measurement
     DevBuf<unsigned long long> computed;
     DevBuf<int> route_list, route_counts;  // the router's per-class FP32 / FP64 / sampled queues
+    DevBuf<int> work_next;  // the Rys kernels' work counters, kCounters a class (KArgs::next)
     // the routed build's budget check (fjb_set_route_check): the FP32 queue's
     // own accumulators, the sample's FP64 and FP32 twins, the verdict
     double check_budget = 1e-8;
@@ -1441,7 +1446,11 @@ void choose_rys(int mode, ClassRun &r) {
         return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
     };
     const auto wtake = [&](bool fp32) {
-        return mode >= 1 && rys_warp_available(la, lb, lc, ld) && (mode == 2 || rys_warp_preferred(la, lb, lc, ld, fp32));
+        // below two units an SM the class's time is one unit's latency: there
+        // the warp kernel's, which spreads a quartet's primitives over lanes,
+        // is the shorter (3-atom build, all classes: 660 -> 562 us)
+        return mode >= 1 && rys_warp_available(la, lb, lc, ld) &&
+               (mode == 2 || rys_warp_preferred(la, lb, lc, ld, fp32) || r.n_units <= 2 * sm_count());
     };
     r.warp64 = wtake(false);
     r.warp32 = wtake(true);
@@ -1699,6 +1708,7 @@ int fjb_plan(fjb_handle *h, const double *D_host, double tau, int n_mag) {
         h->launch_cls.upload(lc);
         h->route_list.alloc(std::max<size_t>(1, 3 * (size_t)h->n_units));
         h->route_counts.alloc(std::max<size_t>(1, 4 * h->runs.size()));
+        h->work_next.alloc(std::max<size_t>(1, kCounters * h->runs.size()));
         if (h->Jp32.n) {  // the budget check's buffers follow the plan's size
             h->Jp32.reset();
             if (int rc = ensure_check(h)) return rc;
@@ -1846,6 +1856,7 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
     CUDA_OK(h, cudaMemsetAsync(h->Jp.p, 0, nn * sizeof(double), st));
     CUDA_OK(h, cudaMemsetAsync(h->Kp.p, 0, nn * sizeof(double), st));
     CUDA_OK(h, cudaMemsetAsync(h->computed.p, 0, h->computed.n * sizeof(unsigned long long), st));
+    CUDA_OK(h, cudaMemsetAsync(h->work_next.p, 0, h->work_next.n * sizeof(int), st));
     const bool routed = route > 0.0;
     h->last_routed = routed;
     const bool check = routed && h->check_budget > 0.0;
@@ -1881,6 +1892,7 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
         CUDA_OK(h, cudaEventRecordWithFlags(h->cev[ri].first, cs, ev_flags));
         KArgs a{};
         a.computed = h->computed.p;
+        a.next = h->work_next.p + kCounters * ri;
         a.C = r.dev;
         a.units = h->units.p + r.unit0;
         a.n_units = r.n_units;
@@ -1926,6 +1938,7 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
             a32.unit_count = cnt;
             a64.unit_list = l64;
             a64.unit_count = cnt + 1;
+            a32.next = a.next + 1;
             if (check) {  // the FP32 queue into its own accumulators
                 a32.Jp = h->Jp32.p;
                 a32.Kp = h->Kp32.p;
@@ -1942,6 +1955,8 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
                 s64.Jp = h->EJ64.p;
                 s64.Kp = h->EK64.p;
                 s32.computed = s64.computed = nullptr;
+                s32.next = a.next + 2;
+                s64.next = a.next + 3;
                 CUDA_OK(h, launch_run32(r, cs, s32));
                 CUDA_OK(h, launch_run(r, cs, s64));
                 launches += 2;
@@ -2000,6 +2015,7 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
             a.boys_tab = h->boys.p;
             a.unit_list = h->route_list.p + r.unit0;
             a.unit_count = h->route_counts.p + 4 * ri + 3;
+            a.next = h->work_next.p + kCounters * ri + 4;
             CUDA_OK(h, launch_run(r, cs, a));
             ++launches;
         }
@@ -3258,7 +3274,7 @@ struct fjb_batch {
     std::vector<ClassRun> runs;
     int n_units = 0, max_nsh = 0;
     size_t max_nn = 0;
-    DevBuf<int> route_list, route_counts;
+    DevBuf<int> route_list, route_counts, work_next;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> cev;
     bool ready = false;  // densities set
@@ -3423,6 +3439,7 @@ int fjb_batch_create(fjb_batch **out, fjb_handle *const *handles, int n) {
         b->bm.alloc(n);
         b->route_list.alloc(std::max<size_t>(1, 2 * (size_t)b->n_units));
         b->route_counts.alloc(std::max<size_t>(1, 4 * b->runs.size()));
+        b->work_next.alloc(std::max<size_t>(1, kCounters * b->runs.size()));
     } catch (const std::exception &e) {
         return bfail(nullptr, FJB_E_CUDA, std::string("fjb_batch_create: ") + e.what());
     }
@@ -3476,6 +3493,7 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
     batch_density_blocks_kernel<<<dim3((unsigned)((b->max_nsh * b->max_nsh + 255) / 256), nm), 256, 0, st>>>(b->bm.p);
     BCUDA_OK(b, cudaMemsetAsync(b->Jp.p, 0, b->Jp.n * sizeof(double), st));
     BCUDA_OK(b, cudaMemsetAsync(b->Kp.p, 0, b->Kp.n * sizeof(double), st));
+    BCUDA_OK(b, cudaMemsetAsync(b->work_next.p, 0, b->work_next.n * sizeof(int), st));
     const bool routed = route > 0.0;
     if (routed) BCUDA_OK(b, cudaMemsetAsync(b->route_counts.p, 0, b->route_counts.n * sizeof(int), st));
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -3502,6 +3520,7 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
         a.boys_tab = h0->boys.p;
         a.mols = b->ctx.p;
         a.launch_mol = b->launch_mol.p;
+        a.next = b->work_next.p + kCounters * ri;
         if (routed) {
             if (!r.has32 && !r.rys32 && !r.warp32)
                 return bfail(b, FJB_E_LIMIT, "fjb_batch_build: a class has no FP32 kernel for routed units");
@@ -3525,6 +3544,7 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
             a32.unit_count = cnt;
             a64.unit_list = l64;
             a64.unit_count = cnt + 1;
+            a32.next = a.next + 1;
             BCUDA_OK(b, launch_run32(r, cs, a32));
             BCUDA_OK(b, launch_run(r, cs, a64));
         } else {

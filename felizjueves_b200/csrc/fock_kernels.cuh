@@ -65,6 +65,9 @@ struct KArgs {
     RysDev Y;
     const double *rys_tab;
     const float *rys_tab32;  // its FP32 copy (the FP32 tier)
+    // the Rys kernels' work counter, zeroed before the build: a warp (CTA) that
+    // finishes its items takes the next ones (null: a static stride)
+    int *next;
     // the batched build: per molecule its context, per launch its molecule
     // (null: one molecule, the fields above)
     const MolCtx *mols;

@@ -62,7 +62,7 @@ cudaError_t rys_launch(int la, int lb, int lc, int ld, bool fp32, int grid, cuda
 
 namespace rys {
 
-constexpr int kItemsPerCta = 6;  // below this many items a CTA, units are cut into slices
+constexpr int kItemsPerCta = 4;  // below this many items a CTA, units are cut into slices
 
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 __host__ __device__ constexpr int nrange(int lo, int hi) {
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
     __shared__ PairRec s_pair[kKetChunk];  // the unit's computed kets, in ket order
     __shared__ int s_oc[kKetChunk], s_od[kKetChunk];
     __shared__ double s_deg[kKetChunk];
-    __shared__ int s_n;
+    __shared__ int s_n, s_next;
     const RysDev &L = A.Y;
     double *braP = sm + L.sm_braP;
     R *cb = reinterpret_cast<R *>(sm + L.sm_cb);
@@ -344,11 +344,14 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
     const int n_todo = A.unit_list ? *A.unit_count : A.n_units;
     // a queue short for the grid: each unit's groups over several CTAs
     const int max_slices = (kKetChunk + G - 1) / G;
-    int ns = n_todo > 0 ? rys::kItemsPerCta * (int)gridDim.x / n_todo : 1;
-    ns = ns < 1 ? 1 : (ns > max_slices ? max_slices : ns);
+    const int want = rys::kItemsPerCta * (int)gridDim.x;
+    int ns = n_todo < want ? (want + n_todo - 1) / max(n_todo, 1) : 1;
+    ns = ns > max_slices ? max_slices : ns;
     const int n_items = n_todo * ns;
+    int taken = 0;
 
-    for (int item_i = blockIdx.x; item_i < n_items; item_i += gridDim.x) {
+    for (int item_i = blockIdx.x; item_i < n_items; item_i = s_next) {
+        if (tid == 0) taken = A.next ? (int)gridDim.x + atomicAdd(A.next, 1) : item_i + (int)gridDim.x;
         const int ui = item_i / ns, slice = item_i - ui * ns;
         const int u = A.unit_list ? A.unit_list[ui] : ui;
         const Unit U = A.units[u];
@@ -631,6 +634,7 @@ __global__ void __launch_bounds__(NT, (rys::Shape<LA, LB, LC, LD>::template minb
         for (int i = tid; i < NAB; i += NT)
             if (Jab[i] != 0.0) red_add(M.Jp + (size_t)(oa + i / NB) * n_ao + ob + i % NB, Jab[i]);
         if (A.computed && tid == 0 && slice == 0 && n_list) atomicAdd(A.computed + U.launch, (unsigned long long)n_list);
+        if (tid == 0) s_next = taken;
         __syncthreads();
     }
 }

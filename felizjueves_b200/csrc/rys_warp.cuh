@@ -38,7 +38,11 @@ namespace rysw {
 
 constexpr int kThreads = 64;  // two independent warps a CTA
 constexpr int kWarps = kThreads / 32;
-constexpr int kItemsPerWarp = 6;  // below this many items a warp, units are cut into slices
+// Below this many items a warp, units are cut into slices.  Items of a class
+// differ by their kets and degrees, so with few a warp the last ones ran on a
+// half-empty chip ((pd|df) at 14 atoms: 3 items a warp, 10 % of 16 % occupancy).
+constexpr int kItemsPerWarp = 4;
+constexpr int kGrabs = 64;  // above this many items a warp, it takes several at a time
 constexpr int kRedSlots = 12;  // FP64 values a lane parks per reduction round
 
 template <int LA, int LB, int LC, int LD, typename R>
@@ -148,17 +152,29 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
     const int n_warps = gridDim.x * rysw::kWarps;
     // a queue short for the grid: each unit's groups over several warps
     constexpr int kMaxSlices = (kKetChunk + GW - 1) / GW;
-    int ns = n_todo > 0 ? rysw::kItemsPerWarp * n_warps / n_todo : 1;
-    ns = ns < 1 ? 1 : (ns > kMaxSlices ? kMaxSlices : ns);
+    const int want = rysw::kItemsPerWarp * n_warps;
+    int ns = n_todo < want ? (want + n_todo - 1) / max(n_todo, 1) : 1;
+    ns = ns > kMaxSlices ? kMaxSlices : ns;
     const int n_items = n_todo * ns;
+    const int grab = max(1, n_items / (n_warps * rysw::kGrabs));
 
     // this lane's bra Cartesian (phases B, C)
     const int gl = lane / NBE, el = lane - gl * NBE;
     int ex = 0, ey = 0, ez = 0;
     rys::cart_of<LA, E>(el, &ex, &ey, &ez);
 
-    for (int it = blockIdx.x * rysw::kWarps + wl; it < n_items; it += n_warps) {
-        const int ui = it / ns, slice = it - ui * ns;
+    int left = 0, taken = 0;  // items left of the warp's grab, the next grab's number
+    const int64_t first = (int64_t)(blockIdx.x * rysw::kWarps + wl) * grab;
+    for (int64_t it = first; it < n_items;
+         it = left > 0 ? it + 1
+                       : (A.next ? (int64_t)(n_warps + __shfl_sync(kAll, taken, 0)) * grab
+                                 : it + (int64_t)n_warps * grab - (grab - 1))) {
+        if (left == 0) {
+            left = grab;
+            if (A.next && lane == 0) taken = atomicAdd(A.next, 1);  // read when the grab is done
+        }
+        --left;
+        const int ui = (int)(it / ns), slice = (int)(it - (int64_t)ui * ns);
         const int u = A.unit_list ? A.unit_list[ui] : ui;
         const Unit U = A.units[u];
         const LaunchRec LR = A.launches[U.launch];
@@ -494,11 +510,15 @@ struct RysWarpOne {
         cudaFuncSetAttribute(rys_warp_kernel<LA, LB, LC, LD, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         done = true;
     }
-    static int occupancy() {
-        attr();
-        int n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_warp_kernel<LA, LB, LC, LD, R>, rysw::kThreads, kSmem);
-        return n;
+    static int occupancy() {  // a constant of the kernel: asked once
+        static const int per_sm = [] {
+            attr();
+            int n = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_warp_kernel<LA, LB, LC, LD, R>, rysw::kThreads,
+                                                          kSmem);
+            return n;
+        }();
+        return per_sm;
     }
     static cudaError_t launch(int grid, cudaStream_t st, const KArgs &a) {
         attr();
