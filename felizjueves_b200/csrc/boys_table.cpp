@@ -20,7 +20,7 @@
 namespace fjb {
 
 std::vector<double> boys_table() {
-    std::vector<double> tab((size_t)kBoysNT * kBoysRow);
+    std::vector<double> tab((size_t)kBoysSize, 0.0);
     for (int i = 0; i < kBoysNT; ++i) {
         long double T = (long double)((double)i * kBoysDelta);  // the node the device uses
         long double ex = expl(-T);
@@ -34,6 +34,11 @@ std::vector<double> boys_table() {
             tab[(size_t)i * kBoysRow + m] = (double)(ex * sum);
         }
         tab[(size_t)i * kBoysRow + kBoysMaxM + 1] = (double)ex;
+        for (int M = 0; M < kBoysOrders; ++M) {  // the rows by order
+            double *row = tab.data() + kBoysByOrder + ((size_t)M * kBoysNT + i) * 8;
+            for (int k = 0; k < kBoysTaylor; ++k) row[k] = tab[(size_t)i * kBoysRow + M + k];
+            row[7] = (double)ex;
+        }
     }
     return tab;
 }

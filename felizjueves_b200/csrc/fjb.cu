@@ -1480,7 +1480,8 @@ int finish_create(std::unique_ptr<fjb_handle> &h, fjb_handle **out) {
     }
     if (cudaSetDevice(device) != cudaSuccess) return fail(nullptr, FJB_E_CUDA, "cudaSetDevice failed");
     try {
-        h->boys.upload(boys_table());
+        static const std::vector<double> boys = boys_table();
+        h->boys.upload(boys);
         h->rys.upload(rys_tables_cached().t64);
         h->rys32.upload(rys_tables_cached().t32);
         std::vector<int> off(h->basis.offsets), nc;

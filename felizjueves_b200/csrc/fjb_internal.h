@@ -19,6 +19,13 @@ constexpr double kBoysDelta = 0.05;
 constexpr double kBoysTMax = 40.0;  // table covers [0, kBoysTMax]
 constexpr int kBoysNT = 801;        // kBoysTMax / kBoysDelta + 1
 constexpr int kBoysRow = kBoysMaxM + 2;  // F_0 .. F_kBoysMaxM, then exp(-T_i)
+// The same table by order, for the kernels whose order M is a compile-time
+// constant: row (M, i) holds F_M .. F_{M+6} and exp(-T_i), 64 aligned bytes
+// read as four vectors from one line where kBoysRow's layout took eight loads
+// from up to three.
+constexpr int kBoysOrders = kMaxLQuartet + 1;
+constexpr int kBoysByOrder = (kBoysNT * kBoysRow + 7) / 8 * 8;  // its offset
+constexpr int kBoysSize = kBoysByOrder + kBoysOrders * kBoysNT * 8;
 constexpr int kThreads = 128;       // widest CTA of the HGP kernel's default choice
 constexpr int kMaxThreads = 512;    // widest CTA the kernel is instantiated for
 constexpr int kKetChunk = 32;       // ket pairs per work unit (one per lane of a warp)
@@ -51,19 +58,20 @@ struct HCoef {
 // zeta, U = c_a c_b (pi/zeta)^{3/2} exp(-alpha beta/zeta |AB|^2), and
 // h = 1/(2 zeta) (the VRR's e/(2 zeta) factor, so no primitive quartet
 // divides by zeta); 80 bytes.
-struct PrimRec {
+struct alignas(16) PrimRec {
     double P[3], X[3], zeta, U, h, pad;
 };
 constexpr int kPrimWords = 10;  // doubles per PrimRec
 static_assert(sizeof(PrimRec) == kPrimWords * sizeof(double), "PrimRec is kPrimWords doubles");
 
 // A contracted shell pair (canonical: la <= lb, lower index first on a tie).
-struct PairRec {
+struct alignas(16) PairRec {
     int32_t a, b, ao_a, ao_b;
     int32_t prim0, nprim, pad0, pad1;
     double G;
     double AB[3];
 };
+static_assert(sizeof(PairRec) == 64 && sizeof(PairRec) % alignof(PairRec) == 0, "PairRec is four 16-byte vectors");
 
 // One launch: a bra batch against a ket batch (bra <= ket).
 struct LaunchRec {
@@ -73,7 +81,7 @@ struct LaunchRec {
 };
 
 // A work unit: bra pair ib of launch `launch`, ket pairs [k0, k1).
-struct Unit {
+struct alignas(16) Unit {
     int32_t launch, ib, k0, k1;
 };
 

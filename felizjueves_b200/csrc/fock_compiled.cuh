@@ -47,18 +47,19 @@ __device__ __forceinline__ void boys_t(double T, double *F, const double *__rest
     if (T < kBoysTMax) {
         const int i = __double2int_rn(T * (1.0 / kBoysDelta));
         const double d = (double)i * kBoysDelta - T;
-        const double *row0 = tab + (size_t)i * kBoysRow;
-        const double *row = row0 + M;
-        double f = __ldg(row + 6);
-        f = __ldg(row + 5) + f * d * (1.0 / 6.0);
-        f = __ldg(row + 4) + f * d * (1.0 / 5.0);
-        f = __ldg(row + 3) + f * d * (1.0 / 4.0);
-        f = __ldg(row + 2) + f * d * (1.0 / 3.0);
-        f = __ldg(row + 1) + f * d * (1.0 / 2.0);
-        f = __ldg(row + 0) + f * d;
+        static_assert(M < kBoysOrders && kBoysTaylor == 7, "a row by order is 7 Taylor terms and exp(-T_i)");
+        const double2 *row = reinterpret_cast<const double2 *>(tab + kBoysByOrder + ((size_t)M * kBoysNT + i) * 8);
+        const double2 r0 = __ldg(row), r1 = __ldg(row + 1), r2 = __ldg(row + 2), r3 = __ldg(row + 3);
+        double f = r3.x;
+        f = r2.y + f * d * (1.0 / 6.0);
+        f = r2.x + f * d * (1.0 / 5.0);
+        f = r1.y + f * d * (1.0 / 4.0);
+        f = r1.x + f * d * (1.0 / 3.0);
+        f = r0.y + f * d * (1.0 / 2.0);
+        f = r0.x + f * d;
         F[M] = f;
         if (M > 0) {
-            const double e = boys_exp(row0, d), t2 = 2.0 * T;
+            const double e = boys_exp_at(r3.y, d), t2 = 2.0 * T;
 #pragma unroll
             for (int m = M - 1; m >= 0; --m) F[m] = (t2 * F[m + 1] + e) * (1.0 / (double)(2 * m + 1));
         }

@@ -100,9 +100,8 @@ __device__ __forceinline__ double *ket_slots(const KArgs &A, int launch, int n_k
 static __constant__ double kRecipOdd[kBoysMaxM + 1] = {1.0 / 1.0, 1.0 / 3.0, 1.0 / 5.0, 1.0 / 7.0, 1.0 / 9.0, 1.0 / 11.0, 1.0 / 13.0, 1.0 / 15.0, 1.0 / 17.0, 1.0 / 19.0, 1.0 / 21.0, 1.0 / 23.0, 1.0 / 25.0, 1.0 / 27.0, 1.0 / 29.0, 1.0 / 31.0, 1.0 / 33.0, 1.0 / 35.0, 1.0 / 37.0, 1.0 / 39.0, 1.0 / 41.0, 1.0 / 43.0, 1.0 / 45.0, 1.0 / 47.0, 1.0 / 49.0};
 
 // exp(-T) at a table node's offset d = T_i - T (|d| <= kBoysDelta/2):
-// exp(-T_i) (the row's last entry) times the degree-8 Taylor polynomial of
-// exp(d), by Horner.
-__device__ __forceinline__ double boys_exp(const double *__restrict__ row0, double d) {
+// exp(-T_i) = e0 times the degree-8 Taylor polynomial of exp(d), by Horner.
+__device__ __forceinline__ double boys_exp_at(double e0, double d) {
     double p = 1.0 / 40320.0;
     p = 1.0 / 5040.0 + d * p;
     p = 1.0 / 720.0 + d * p;
@@ -112,7 +111,11 @@ __device__ __forceinline__ double boys_exp(const double *__restrict__ row0, doub
     p = 0.5 + d * p;
     p = 1.0 + d * p;
     p = 1.0 + d * p;
-    return __ldg(row0 + kBoysMaxM + 1) * p;
+    return e0 * p;
+}
+// the same from a table row, its last entry
+__device__ __forceinline__ double boys_exp(const double *__restrict__ row0, double d) {
+    return boys_exp_at(__ldg(row0 + kBoysMaxM + 1), d);
 }
 
 __device__ __forceinline__ void boys_eval(int M, double T, double *F, const double *__restrict__ tab) {
