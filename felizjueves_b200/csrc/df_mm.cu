@@ -111,20 +111,65 @@ __device__ __forceinline__ void split3(double v, __nv_bfloat16 *h, __nv_bfloat16
 //   mode 0: src[r * ld + c]
 //   mode 1: src[(c / n) * n * n + r * n + c % n]  (the aux-batched
 //           transpose: row r of every n x n block q, side by side)
-__global__ void df_split_kernel(const double *__restrict__ src, int mode, long long rows, long long cols,
-                                long long ld, long long n, long long rows_p, long long ldp, __nv_bfloat16 *hi,
-                                __nv_bfloat16 *mid, __nv_bfloat16 *lo) {
-    const long long total = rows_p * ldp, kts = ldp / kMmK;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long tile = i >> 13, w = i & 8191;
+// A CTA a tile, 64 rows at a time: a warp reads a row's 64 values two a lane
+// (the lane's columns, and their block and place in mode 1, are the same for
+// every row), the parts go to shared memory by rows and leave as whole 16-byte
+// core-matrix rows in the tile's order.  HBM-bound: 8 bytes read and 6 written
+// an element.
+constexpr int kSplitThreads = 256, kSplitRows = 64, kSplitStride = kMmK + 8;  // rows 144 bytes apart: no bank conflict
+
+__global__ void __launch_bounds__(kSplitThreads)
+    df_split_kernel(const double *__restrict__ src, int mode, long long rows, long long cols, long long ld,
+                    long long n, long long rows_p, long long ldp, __nv_bfloat16 *hi, __nv_bfloat16 *mid,
+                    __nv_bfloat16 *lo) {
+    __shared__ __align__(16) __nv_bfloat16 part[3][kSplitRows * kSplitStride];
+    const long long kts = ldp / kMmK, tiles = (rows_p / kMmTile) * kts;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = kSplitThreads / 32, kPer = kSplitRows / kWarps;
+    const long long rs = mode == 0 ? ld : n;
+    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const long long rt = tile / kts, kt = tile - rt * kts;
-        const int rem = (int)(w & 511), r8 = (int)(w >> 9);
-        const long long r = rt * kMmTile + r8 * 8 + ((rem & 63) >> 3);
-        const long long c = kt * kMmK + (rem >> 6) * 8 + (rem & 7);
-        double v = 0.0;
-        if (r < rows && c < cols) v = mode == 0 ? src[r * ld + c] : src[(c / n) * n * n + r * n + c % n];
-        split3(v, hi + i, mid + i, lo + i);
+        const long long c0 = kt * kMmK + 2 * lane, c1 = c0 + 1;
+        long long o0 = c0, o1 = c1;
+        if (mode != 0) {
+            const long long q0 = c0 / n, j0 = c0 - q0 * n;
+            o0 = q0 * n * n + j0;
+            o1 = j0 + 1 < n ? o0 + 1 : (q0 + 1) * n * n;
+        }
+        for (int half = 0; half < kMmTile / kSplitRows; ++half) {
+            const long long r0 = rt * kMmTile + half * kSplitRows + warp * kPer;
+            double v0[kPer], v1[kPer];
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+                const double *row = src + (r0 + k) * rs;
+                const bool in = r0 + k < rows;
+                v0[k] = in && c0 < cols ? row[o0] : 0.0;
+                v1[k] = in && c1 < cols ? row[o1] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+                __nv_bfloat162 h, m, l;
+                split3(v0[k], &h.x, &m.x, &l.x);
+                split3(v1[k], &h.y, &m.y, &l.y);
+                const int at = (warp * kPer + k) * kSplitStride + 2 * lane;
+                *reinterpret_cast<__nv_bfloat162 *>(&part[0][at]) = h;
+                *reinterpret_cast<__nv_bfloat162 *>(&part[1][at]) = m;
+                *reinterpret_cast<__nv_bfloat162 *>(&part[2][at]) = l;
+            }
+            __syncthreads();
+            constexpr int kUnits = kSplitRows * kMmK / 8;  // 16-byte core-matrix rows a part
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                __nv_bfloat16 *out = (x == 0 ? hi : (x == 1 ? mid : lo)) + tile * (kMmTile * kMmK) +
+                                     half * (kSplitRows * kMmK);
+                for (int i = threadIdx.x; i < kUnits; i += kSplitThreads) {
+                    const int r = (i >> 6) * 8 + (i & 7), kg = (i >> 3) & 7;
+                    reinterpret_cast<uint4 *>(out)[i] =
+                        *reinterpret_cast<const uint4 *>(&part[x][r * kSplitStride + kg * 8]);
+                }
+            }
+            __syncthreads();
+        }
     }
 }
 
@@ -303,15 +348,29 @@ __global__ void df_gamma_kernel(const double *__restrict__ B, const double *__re
     }
 }
 
-// J[i] = sum_q B[q][i] gamma_q (FP64): a thread per element, q in order
-// (coalesced across i).
-__global__ void df_jmat_kernel(const double *__restrict__ B, const double *__restrict__ gamma, long long nq,
-                               long long nn, double *J) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nn;
-         i += (long long)gridDim.x * blockDim.x) {
+// J[i] = sum_q B[q][i] gamma_q (FP64): 64 elements a CTA, coalesced across i,
+// the aux functions in eight interleaved sums (one thread an element kept too
+// few loads in flight: 186 us for 354 MB at 248 AO and 720 aux functions).
+constexpr int kJmatCols = 64, kJmatRows = 8;
+__global__ void __launch_bounds__(kJmatCols *kJmatRows)
+    df_jmat_kernel(const double *__restrict__ B, const double *__restrict__ gamma, long long nq, long long nn,
+                   double *J) {
+    __shared__ double part[kJmatRows][kJmatCols];
+    for (long long i0 = (long long)blockIdx.x * kJmatCols; i0 < nn; i0 += (long long)gridDim.x * kJmatCols) {
+        const long long i = i0 + threadIdx.x;
         double s = 0.0;
-        for (long long q = 0; q < nq; ++q) s += B[q * nn + i] * gamma[q];
-        J[i] = s;
+        if (i < nn) {
+#pragma unroll 6
+            for (long long q = threadIdx.y; q < nq; q += kJmatRows) s += B[q * nn + i] * gamma[q];
+        }
+        part[threadIdx.y][threadIdx.x] = s;
+        __syncthreads();
+        if (threadIdx.y == 0 && i < nn) {
+#pragma unroll
+            for (int k = 1; k < kJmatRows; ++k) s += part[k][threadIdx.x];
+            J[i] = s;
+        }
+        __syncthreads();
     }
 }
 
@@ -399,21 +458,22 @@ cudaError_t df_jk_launch(const double *B, long long nq, long long n, const doubl
         static_cast<unsigned char *>(work) + round_up((round_up(nq, 32) + nq * n * n) * (long long)sizeof(double), 256));
     const long long nn = n * n;
     df_gamma_kernel<<<(unsigned)nq, 256, 0, st>>>(B, D, nn, gamma);
-    df_jmat_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(B, gamma, nq, nn, J);
+    df_jmat_kernel<<<(unsigned)((nn + kJmatCols - 1) / kJmatCols), dim3(kJmatCols, kJmatRows), 0, st>>>(B, gamma, nq, nn,
+                                                                                                     J);
     // GEMM 1: X (nq n x n) = B (nq n x n) . D^T (D symmetric)
     __nv_bfloat16 *a1 = sp, *b1 = sp + 3 * s.rows1 * s.ld1;
-    const unsigned sgrid = 148 * 16;
-    df_split_kernel<<<sgrid, 256, 0, st>>>(B, 0, nq * n, n, n, n, s.rows1, s.ld1, a1, a1 + s.rows1 * s.ld1,
+    const unsigned sgrid = 148 * 8;
+    df_split_kernel<<<sgrid, kSplitThreads, 0, st>>>(B, 0, nq * n, n, n, n, s.rows1, s.ld1, a1, a1 + s.rows1 * s.ld1,
                                            a1 + 2 * s.rows1 * s.ld1);
-    df_split_kernel<<<sgrid, 256, 0, st>>>(D, 0, n, n, n, n, s.rowsn, s.ld1, b1, b1 + s.rowsn * s.ld1,
+    df_split_kernel<<<sgrid, kSplitThreads, 0, st>>>(D, 0, n, n, n, n, s.rowsn, s.ld1, b1, b1 + s.rowsn * s.ld1,
                                            b1 + 2 * s.rowsn * s.ld1);
     cudaError_t e = df_mm(a1, s.rows1, b1, s.rowsn, s.ld1, nq * n, n, X, n, err, st);
     if (e != cudaSuccess) return e;
     // GEMM 2: K (n x n) = [X_q rows side by side] . [B_q rows side by side]^T
     __nv_bfloat16 *a2 = sp, *b2 = sp + 3 * s.rowsn * s.ld2;
-    df_split_kernel<<<sgrid, 256, 0, st>>>(X, 1, n, nq * n, 0, n, s.rowsn, s.ld2, a2, a2 + s.rowsn * s.ld2,
+    df_split_kernel<<<sgrid, kSplitThreads, 0, st>>>(X, 1, n, nq * n, 0, n, s.rowsn, s.ld2, a2, a2 + s.rowsn * s.ld2,
                                            a2 + 2 * s.rowsn * s.ld2);
-    df_split_kernel<<<sgrid, 256, 0, st>>>(B, 1, n, nq * n, 0, n, s.rowsn, s.ld2, b2, b2 + s.rowsn * s.ld2,
+    df_split_kernel<<<sgrid, kSplitThreads, 0, st>>>(B, 1, n, nq * n, 0, n, s.rowsn, s.ld2, b2, b2 + s.rowsn * s.ld2,
                                            b2 + 2 * s.rowsn * s.ld2);
     e = df_mm(a2, s.rowsn, b2, s.rowsn, s.ld2, n, n, K, n, err, st);
     if (e != cudaSuccess) return e;
@@ -433,7 +493,7 @@ cudaError_t df_syrk_launch(const double *Z, long long rows, long long cols, doub
                            cudaStream_t st) {
     const long long rp = round_up(rows, kMmTile), ldp = round_up(cols, kMmK);
     __nv_bfloat16 *a = static_cast<__nv_bfloat16 *>(work);
-    df_split_kernel<<<148 * 16, 256, 0, st>>>(Z, 0, rows, cols, cols, 0, rp, ldp, a, a + rp * ldp, a + 2 * rp * ldp);
+    df_split_kernel<<<148 * 8, kSplitThreads, 0, st>>>(Z, 0, rows, cols, cols, 0, rp, ldp, a, a + rp * ldp, a + 2 * rp * ldp);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = df_mm(a, rp, a, rp, ldp, rows, rows, K, rows, err, st, 256);
