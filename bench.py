@@ -424,14 +424,12 @@ def main():
                    "l2": "working set > 126 MB L2 (6 x 31.5 MB matrices + pair records); no flush"},
         "roofline": {"bound": "fp64",
                      "kernel": "%s class (%d%d|%d%d)" % (("hgp_fock_kernel", "hgp_compiled_kernel",
-                                                          "rys_fock_kernel")[top.get("engine", 0)], *tcls),
+                                                          "rys_warp_kernel")[top.get("engine", 0)], *tcls),
                      "achieved": round(ach, 3), "peak": round(peak64, 3), "unit": "TFLOP/s",
                      "frac": round(ach / peak64, 4) if peak64 else None, "traffic": None,
-                     "traffic_note": "not captured at this size; the kernel is FP64-issue and "
-                                     "latency bound, its pair records and D read from L2: ncu "
-                                     "measured 1.6 MB read + 23 MB written per launch of the "
-                                     "(pp|pf) Rys class on a 16-atom cluster "
-                                     "(profiles/rys_fock_kernel_pppf_cluster16.md)",
+                     "traffic_note": "not captured at this size; the kernel is latency- and "
+                                     "shared-memory-bound, its pair records and D read from L2 "
+                                     "(profiles/rys_warp_kernel_cluster14.md)",
                      "peak_source": "measured: fjb_fma_probe FP64 FMA chains on this GPU "
                                     "(MEASURED_PEAKS.json has no FP64 figure)",
                      "build_tflops": round(build_tf, 3), "kernel_ms": round(top["ms"], 3),

@@ -27,10 +27,10 @@ OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "libfjb.so")
 REPO = os.path.dirname(HERE)
 
-CU_SOURCES = ["fjb.cu", "fock_compiled.cu", "router.cu", "jengine.cu", "onee.cu", "rys_fock.cu",
-              "rys_fock64.cu", "rys_fock32.cu", "df_mm.cu", "df_eri3.cu", "rys_warp.cu", "jrys.cu"]
+CU_SOURCES = ["fjb.cu", "fock_compiled.cu", "router.cu", "jengine.cu", "onee.cu",
+              "df_mm.cu", "df_eri3.cu", "rys_warp.cu", "jrys.cu"]
 # rys_warp_inst.cu, once per bra class and precision (rys_warp.h's lists)
-RYS_WARP_PARTS = [(p, f) for p in ("SD", "SF", "SP", "PP", "PD", "DD") for f in (0, 1)]
+RYS_WARP_PARTS = [(p, f) for p in ("DF", "PF", "SD", "SF", "SP", "PP", "PD", "DD") for f in (0, 1)]
 CPP_SOURCES = ["plan.cpp", "hgp_tables.cpp", "boys_table.cpp", "scatter.cpp", "rys_table.cpp", "hjk_plan.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -19,14 +19,14 @@
 //      (a, b), at [m][n][P] and, for a != b, at the mirror [n][m][P]; the
 //      threads of one aux shell and its neighbours write consecutive P.
 //
-// The same recurrences and rule as the Rys Fock kernel (rys_fock.cuh), in
+// The same recurrences and rule as the Rys Fock kernel (rys_warp.cuh), in
 // FP64.  la >= lb puts the larger shell on the transfer's receiving side,
 // so (f s|P) needs no HRR at all.
 #pragma once
 #include <cuda_runtime.h>
 
 #include "fjb_internal.h"
-#include "rys_fock.cuh"
+#include "rys_device.cuh"
 
 // The classes (la >= lb, both <= 3; aux l <= 4)
 #define FJB_E3_BRAS(X, LP) \

@@ -29,7 +29,7 @@
 #include "plan.h"
 #include "scatter.h"
 #include "router.cuh"
-#include "rys_fock.cuh"
+#include "rys_device.cuh"
 #include "rys_warp.h"
 #include "side_streams.h"
 #include "df_eri3.cuh"
@@ -901,14 +901,10 @@ struct ClassEntry {
 
 struct ClassRun {
     ClassDev dev;  // the interpreter kernel's layout (kept valid for every class)
-    // the Rys kernel (rys_fock.cuh) for this class's FP64 / FP32 units, when
-    // it takes the class: its carve-up, grid and the tabulated rule it reads
+    // the Rys kernel (rys_warp.cuh) for this class's FP64 / FP32 units, when it
+    // takes the class: its grid and the tabulated rule it reads
     bool rys64 = false, rys32 = false;
-    RysDev ry64{}, ry32{};
     int grid_r64 = 0, grid_r32 = 0;
-    // the warp-autonomous Rys kernel (rys_warp.cuh), when it takes the class
-    bool warp64 = false, warp32 = false;
-    int grid_w64 = 0, grid_w32 = 0;
     const double *rys_tab = nullptr;
     const float *rys_tab32 = nullptr;
     ClassDev dev32;  // the FP32 interpreter's layout (routed builds of classes without has32)
@@ -954,41 +950,27 @@ int sm_count() {
 // warps to a CTA; the interpreter one CTA on a unit.
 int run_grid(const ClassRun &r);
 
-// The FP64 path of a class run: its register kernel, else the Rys kernel,
-// else the interpreter (which alone serves the atomics-free build's slots).
+// The FP64 path of a class run: the Rys kernel where it takes the class, else
+// its register kernel, else the interpreter (which alone serves the atomics-free build's slots).
 cudaError_t launch_run(const ClassRun &r, cudaStream_t st, const KArgs &a) {
-    if (r.warp64 && !a.W) {
-        KArgs ar = a;
-        ar.rys_tab = r.rys_tab;
-        return rys_warp_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, false, r.grid_w64, st, ar);
-    }
     if (r.rys64 && !a.W) {
         KArgs ar = a;
-        ar.Y = r.ry64;
         ar.rys_tab = r.rys_tab;
-        ar.rys_tab32 = r.rys_tab32;
-        return rys_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, false, r.grid_r64, st, ar);
+        return rys_warp_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, false, r.grid_r64, st, ar);
     }
     if (r.compiled) return launch_compiled(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, false, r.grid, st, a);
     return launch_hgp<double>(r.dev, r.grid, st, a);
 }
 
-// The FP32 kernel of a class run (routed builds): its register kernel, else
-// the Rys kernel in FP32, else the interpreter in FP32 with its own layout.
+// The FP32 kernel of a class run (routed builds): the Rys kernel in FP32 where
+// it takes the class, else its register kernel, else the interpreter in FP32 with its own layout.
 cudaError_t launch_run32(const ClassRun &r, cudaStream_t st, const KArgs &a) {
-    if (r.warp32 && !a.W) {
-        KArgs ar = a;
-        ar.rys_tab32 = r.rys_tab32;
-        return rys_warp_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid_w32, st, ar);
-    }
-    if (r.has32) return launch_compiled(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid32, st, a);
     if (r.rys32 && !a.W) {
         KArgs ar = a;
-        ar.Y = r.ry32;
-        ar.rys_tab = r.rys_tab;
         ar.rys_tab32 = r.rys_tab32;
-        return rys_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid_r32, st, ar);
+        return rys_warp_launch(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid_r32, st, ar);
     }
+    if (r.has32) return launch_compiled(r.dev.la, r.dev.lb, r.dev.lc, r.dev.ld, true, r.grid32, st, a);
     KArgs a32 = a;
     a32.C = r.dev32;
     return launch_hgp<float>(r.dev32, r.grid32, st, a32);
@@ -1424,38 +1406,25 @@ int append_shells(fjb_handle *h, const fjb_basis *b, int max_l) {
 // sizes, the build events.
 // Which kernels a class run's units take from the Rys kernel: mode 0 none;
 // 0 none; 1 the classes without an FP64 (FP32) register body and those where
-// the Rys kernel is the faster; 2 every class it has.  Bras of at most 32
-// Cartesians run on the warp kernel (rys_warp.cuh), the longer ones on the
-// CTA kernel (rys_fock.cuh).
+// the Rys kernel is the faster; 2 every class it has.
 void choose_rys(int mode, ClassRun &r) {
     const int la = r.dev.la, lb = r.dev.lb, lc = r.dev.lc, ld = r.dev.ld;
-    r.rys64 = mode >= 1 && rys_available(la, lb, lc, ld) &&
-              rys_layout(la, lb, lc, ld, r.max_kab, r.max_kcd, false, kSmemBudgetDoubles, &r.ry64);
-    r.rys32 = mode >= 1 && rys_available(la, lb, lc, ld) &&
-              rys_layout(la, lb, lc, ld, r.max_kab, r.max_kcd, true, kSmemBudgetDoubles, &r.ry32);
-    const auto rgrid = [&](bool fp32, const RysDev &d) {
-        const int per_sm = std::max(1, rys_blocks_per_sm(la, lb, lc, ld, fp32, d));
-        const int64_t most = (int64_t)r.n_units * ((kKetChunk + d.group - 1) / d.group);  // a slice a group
-        return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
-    };
-    if (r.rys64) r.grid_r64 = rgrid(false, r.ry64);
-    if (r.rys32) r.grid_r32 = rgrid(true, r.ry32);
-    const auto wgrid = [&](bool fp32) {
+    const auto grid = [&](bool fp32) {
         const int64_t most = (int64_t)r.n_units * kKetChunk;  // a unit makes at most one item a ket
         const int per_sm = std::max(1, rys_warp_blocks_per_sm(la, lb, lc, ld, fp32));
         return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
     };
-    const auto wtake = [&](bool fp32) {
+    const auto take = [&](bool fp32) {
         // below two units an SM the class's time is one unit's latency: there
-        // the warp kernel's, which spreads a quartet's primitives over lanes,
+        // the Rys kernel's, which spreads a quartet's primitives over lanes,
         // is the shorter (3-atom build, all classes: 660 -> 562 us)
         return mode >= 1 && rys_warp_available(la, lb, lc, ld) &&
                (mode == 2 || rys_warp_preferred(la, lb, lc, ld, fp32) || r.n_units <= 2 * sm_count());
     };
-    r.warp64 = wtake(false);
-    r.warp32 = wtake(true);
-    if (r.warp64) r.grid_w64 = wgrid(false);
-    if (r.warp32) r.grid_w32 = wgrid(true);
+    r.rys64 = take(false);
+    r.rys32 = take(true);
+    if (r.rys64) r.grid_r64 = grid(false);
+    if (r.rys32) r.grid_r32 = grid(true);
 }
 
 // The Rys rule's device tables, FP64 and FP32, built once per process
@@ -3448,7 +3417,7 @@ int fjb_batch_create(fjb_batch **out, fjb_handle *const *handles, int n) {
         choose_rys(1, r);
         r.grid = run_grid(r);
         r.grid32 = run_grid32(r);
-        if (!r.compiled && !r.rys64 && !r.warp64)
+        if (!r.compiled && !r.rys64)
             return bfail(nullptr, FJB_E_LIMIT, "fjb_batch_create: a class has neither a register nor a Rys kernel");
         cudaEvent_t e0, e1;
         if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
@@ -3523,7 +3492,7 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
         a.launch_mol = b->launch_mol.p;
         a.next = b->work_next.p + kCounters * ri;
         if (routed) {
-            if (!r.has32 && !r.rys32 && !r.warp32)
+            if (!r.has32 && !r.rys32)
                 return bfail(b, FJB_E_LIMIT, "fjb_batch_build: a class has no FP32 kernel for routed units");
             int *l32 = b->route_list.p + r.unit0;
             int *l64 = b->route_list.p + b->n_units + r.unit0;

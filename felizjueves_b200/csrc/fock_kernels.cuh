@@ -61,11 +61,10 @@ struct KArgs {
     const int64_t *w_base;   // per launch: its first slot in W
     double *wab;             // per unit: the bra block's partial sums
     const int64_t *wab_off;  // per unit of this run: its offset in wab
-    // the Rys kernel (rys_fock.cuh): its layout and the tabulated rule
-    RysDev Y;
+    // the Rys kernel (rys_warp.cuh): the tabulated rule
     const double *rys_tab;
     const float *rys_tab32;  // its FP32 copy (the FP32 tier)
-    // the Rys kernels' work counter, zeroed before the build: a warp (CTA) that
+    // the Rys kernel's work counter, zeroed before the build: a team that
     // finishes its items takes the next ones (null: a static stride)
     int *next;
     // the batched build: per molecule its context, per launch its molecule

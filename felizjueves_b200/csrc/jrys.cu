@@ -22,7 +22,7 @@
 // bound: lp, lq = 3, 4 is 390 FMAs a root for 35 shared loads.
 #include "jrys.h"
 
-#include "rys_fock.cuh"
+#include "rys_device.cuh"
 
 namespace fjb {
 

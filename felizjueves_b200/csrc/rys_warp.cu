@@ -1,10 +1,12 @@
-// rys_warp.cu -- host dispatch of the warp-autonomous Rys kernel
+// rys_warp.cu -- host dispatch of the Rys Fock kernel
 // (rys_warp.cuh; its instantiations: rys_warp_inst.cu).
 #include "rys_warp.h"
 
 #include "fock_kernels.cuh"
 
 namespace fjb {
+
+bool compiled_available(int la, int lb, int lc, int ld, bool fp32);  // fock_compiled.cu
 
 #define FJB_X(a, b, c, d)                                                         \
     int rys_warp_occ64_##a##b##c##d();                                            \
@@ -37,7 +39,7 @@ bool rys_warp_preferred(int la, int lb, int lc, int ld, bool fp32) {
         return n;
     };
     const int e = rows(la, lb), f = rows(lc, ld);
-    return e * f > 100 && !(fp32 && f < e);
+    return e * f > 100 && !(fp32 && f < e && compiled_available(la, lb, lc, ld, true));
 }
 
 int rys_warp_blocks_per_sm(int la, int lb, int lc, int ld, bool fp32) {

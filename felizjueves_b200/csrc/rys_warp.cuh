@@ -1,14 +1,16 @@
-// rys_warp.cuh -- the warp-autonomous Rys Fock kernel.
+// rys_warp.cuh -- the Rys Fock kernel.
 //
-// rys_warp_kernel<LA, LB, LC, LD, R>: one WARP per work item (a work unit --
-// a bra shell pair and up to 32 of its kets -- or, when the queue is shorter
-// than the grid, a slice of one), the item's computed kets taken GW at a
-// time.  No CTA barrier anywhere: the phases of a warp are ordered by
-// __syncwarp, and the other warps of the SM fill its latencies.  Per group:
+// rys_warp_kernel<LA, LB, LC, LD, R>: a team of threads per work item (a work
+// unit -- a bra shell pair and up to 32 of its kets -- or, when the queue is
+// short for the grid, a slice of one), the item's computed kets taken GW at a
+// time.  The team is one WARP where the bra's row of Cartesians fits a warp
+// (to dd: 31): then there is no CTA barrier anywhere, the phases are ordered
+// by __syncwarp and the other warps of the SM fill the latencies.  The pf, df
+// and ff bras (34, 52, 74) take a CTA of 128, 64 and 96.  Per group of kets:
 //
 //   A  tables: a lane per (ket, primitive quartet x root): the Rys rule at T
 //      (rys_rule.h) and the three axes' 2D integrals I(i, k), the root's
-//      weight and the seed folded into z, into the warp's shared memory; CH
+//      weight and the seed folded into z, into the team's shared memory; CH
 //      (quartet, root) entries of each ket a round.
 //   B  boundary: a lane per (ket, e), e a bra Cartesian of la <= |e| <= la +
 //      lb, holds the whole ket row [e0|f0] for every f with lc <= |f| <= lc +
@@ -23,42 +25,60 @@
 //      and forms J_cd, its shares of K_ad, K_bd (summed over c) and of K_ac,
 //      K_bc (summed over d through shared memory); FP64 throughout.
 //
-// Why this split: with the kets' f in lanes and the bra's e in registers
-// (rys_fock.cuh) a short bra leaves 1.2 FP64 operations per double read from
-// shared memory -- 15 per 12 for (pp|pf) -- and the phase runs at the shared
-// memory's rate; the longer ket side in registers makes it 49 per 15.  The
-// CTA kernel's other half went to its barriers and to staging one unit at a
-// time per CTA.
+// This is the reference's third engine (rys/, eri/fock/kernel_frys.py:194)
+// as the VRR of the fused HGP build: the boundary is the same set of values
+// the HGP VRR produces, so the HRR and digest are the build's own.  R = double
+// is the plain FP64 path; R = float the routed path's FP32 tier (the rule,
+// tables, boundary and HRR in FP32; T, the pair scalars, densities and every
+// J/K accumulation FP64).
+//
+// Why this split: with the kets' f in lanes and the bra's e in registers a
+// short bra leaves 1.2 FP64 operations per double read from shared memory --
+// 15 per 12 for (pp|pf) -- and the phase runs at the shared memory's rate;
+// the longer ket side in registers makes it 49 per 15.  A CTA-per-unit kernel
+// of that form spent the rest on barriers and on staging one unit at a time:
+// 32-atom cluster of the 64-atom workload's shells, ms a class, it / this:
+// (pf|df) 16.0 / 6.5, (pf|pf) 13.2 / 5.1, (df|df) 10.2 / 3.0, (df|ff) 9.3 /
+// 2.9; 20 atoms: (pd|pf) 8.7 / 3.8, (sd|pf) 8.0 / 2.4, (pp|pf) 8.1 / 2.3,
+// (sp|ff) 4.4 / 1.3.
+//
+// What bounds it: latency and the shared-memory pipe more than FP64.  ncu on
+// (sd|pf) and (pd|df), 14 atoms: FP64 pipe 24 % and 21 %, shared/L1 data pipe
+// 50 % and 36 %, long scoreboard 4.3 and 2.6 of some 9 and 7 stall cycles an
+// instruction, 16 and 10 warps an SM by registers and shared memory.
 #pragma once
-#include "rys_fock.cuh"
+#include "rys_device.cuh"
 
 namespace fjb {
 
 namespace rysw {
 
-constexpr int kThreads = 64;  // two independent warps a CTA
-constexpr int kWarps = kThreads / 32;
-// Below this many items a warp, units are cut into slices.  Items of a class
+// Below this many items a team, units are cut into slices.  Items of a class
 // differ by their kets and degrees, so with few a warp the last ones ran on a
 // half-empty chip ((pd|df) at 14 atoms: 3 items a warp, 10 % of 16 % occupancy).
-constexpr int kItemsPerWarp = 4;
-constexpr int kGrabs = 64;  // above this many items a warp, it takes several at a time
+constexpr int kItemsPerWarp = 4;  // a team
+constexpr int kGrabs = 64;        // above this many items a team, it takes several at a time
 constexpr int kRedSlots = 12;  // FP64 values a lane parks per reduction round
 
 template <int LA, int LB, int LC, int LD, typename R>
 struct Shape {
     using S = rys::Shape<LA, LB, LC, LD>;
+    // The team of threads that works on an item: a warp where the bra's row
+    // fits one; for pf (34), df (52) and ff (74) the CTA width that wastes
+    // least of its lanes (3 x 34 of 128, 52 of 64, 74 of 96).
+    static constexpr int TW = S::NBE <= 32 ? 32 : (S::NBE == 34 ? 128 : (S::NBE == 52 ? 64 : 96));
+    static constexpr int kThreads = TW == 32 ? 64 : TW;  // two independent warps, or one team, a CTA
+    static constexpr int kTeams = kThreads / TW;
     static constexpr int E = S::E, F = S::F, NR = S::NR;
     static constexpr int NA = S::NA, NB = S::NB, NC = S::NC, ND = S::ND, NAB = S::NAB, NCD = S::NCD;
     static constexpr int NBE = S::NBE, NBF = S::NBF;
-    static constexpr int GW = 32 / NBE;  // kets a group: a lane per (ket, e)
-    static constexpr int CH = 32 / GW;   // table entries of each ket a round: a lane per entry
+    static constexpr int GW = TW / NBE;  // kets a group: a lane per (ket, e)
     static constexpr int TS = (E + 1) * (F + 1);
     static constexpr int STR = (3 * TS) | 1;  // odd: entries start in different banks
     static constexpr int XS = NCD | 1;
     // digest lanes: GX kets x CS residues of c x ND values of d
     static constexpr int cs_of(int gx) {
-        const int n = 32 / (gx * ND);
+        const int n = TW / (gx * ND);
         return n < 1 ? 0 : (n > NC ? NC : n);
     }
     static constexpr int cost(int gx) {
@@ -74,25 +94,34 @@ struct Shape {
     static constexpr int GX = pick_gx(), CS = cs_of(GX), CPL = (NC + CS - 1) / CS;
     static constexpr int NK = NA + NB;  // K columns a lane owns per c
     static constexpr int BATCH = kRedSlots / NK < 1 ? 1 : (kRedSlots / NK > CPL ? CPL : kRedSlots / NK);
-    static constexpr int RED = BATCH * NK * 32;
+    static constexpr int RED = BATCH * NK * TW;
     // a warp's shared memory, in doubles
     static constexpr int wd(int n) { return (n * (int)sizeof(R) + 7) / 8; }
-    static constexpr int TABD = wd(GW * CH * STR), XD = wd(GW * NBE * XS);
+    static constexpr int XD = wd(GW * NBE * XS);
+    // table entries of each ket a round: a lane per entry; the wider teams'
+    // tables no larger than the rows they make room for afterwards
+    static constexpr int ch() {
+        const int most = TW / GW, fit = (XD + RED) / wd(GW * STR);
+        return TW == 32 || fit > most ? most : (fit < 8 ? 8 : fit);
+    }
+    static constexpr int CH = ch();
+    static constexpr int TABD = wd(GW * CH * STR);
     static constexpr int REGION = TABD > XD + RED ? TABD : XD + RED;
-    static constexpr int SMD = REGION + NAB + 32 * 4 + 48;  // + D_ab, the kets' degeneracies, separations, indices
-    // warps an SM: by shared memory, and by the registers of the ket row (16
+    static constexpr int SMD = REGION + NAB + 32 * 4 + 50;  // + D_ab, the kets' degeneracies, separations, indices
+    // CTAs an SM: by shared memory, and by the registers of the ket row (16
     // warps leave 128 a thread, 12 leave 168, 8 leave 255).  At 16 the rows of
     // 30 to 34 doubles spill through phase A: (sd|pf) 2.90 ms against 2.39 at
     // 12, (pp|pf) 2.87 against 2.30; the 16-double row fits, (sf|pd) 3.33
     // against 3.67 (20-atom cluster of the 64-atom workload's shells).
-    static constexpr int warps_smem() { return 232448 / (SMD * 8 + 512); }
+    static constexpr int ctas_smem() { return 232448 / (kTeams * SMD * 8 + 1024); }
     static constexpr int warps_regs() {
         const int row = NBF * (int)sizeof(R);
         return row <= 160 ? 16 : (row <= 52 * 8 ? 12 : 8);
     }
     static constexpr int minb() {
-        const int w = warps_smem() < warps_regs() ? warps_smem() : warps_regs();
-        return w / kWarps < 1 ? 1 : w / kWarps;
+        const int r = warps_regs() * 32 / kThreads;
+        const int n = ctas_smem() < r ? ctas_smem() : r;
+        return n < 1 ? 1 : n;
     }
 };
 
@@ -121,11 +150,12 @@ __device__ __forceinline__ void ld_prim(const PrimRec *__restrict__ p, double *o
 }  // namespace rysw
 
 template <int LA, int LB, int LC, int LD, typename R>
-__global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R>::minb()))
+__global__ void __launch_bounds__((rysw::Shape<LA, LB, LC, LD, R>::kThreads), (rysw::Shape<LA, LB, LC, LD, R>::minb()))
     rys_warp_kernel(const KArgs A) {
     using S = rysw::Shape<LA, LB, LC, LD, R>;
     constexpr int E = S::E, F = S::F, NR = S::NR, GW = S::GW, CH = S::CH, TS = S::TS, STR = S::STR, XS = S::XS;
     constexpr int NA = S::NA, NB = S::NB, NC = S::NC, ND = S::ND, NAB = S::NAB;
+    constexpr int TW = S::TW;
     constexpr int NBE = S::NBE, NBF = S::NBF, GX = S::GX, CS = S::CS, CPL = S::CPL, NK = S::NK, BATCH = S::BATCH;
     constexpr const rys::CSet<LA, E> &es = rys::kCart<LA, E>;
     constexpr const rys::CSet<LC, F> &fs = rys::kCart<LC, F>;
@@ -137,7 +167,13 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
     constexpr unsigned kAll = 0xffffffffu;
 
     extern __shared__ __align__(16) double sm[];
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const int lane = threadIdx.x % TW, wl = threadIdx.x / TW;  // place in the team, team in the CTA
+    const auto sync = [] {
+        if constexpr (TW == 32)
+            __syncwarp();
+        else
+            __syncthreads();
+    };
     double *ws = sm + wl * S::SMD;
     R *tab = reinterpret_cast<R *>(ws);
     R *X = reinterpret_cast<R *>(ws);
@@ -146,32 +182,41 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
     double *s_deg = Dab + NAB;
     double *s_sep = s_deg + 32;  // [3][32]
     int *s_prim = reinterpret_cast<int *>(s_sep + 96);
-    int *s_oc = s_prim + 32, *s_od = s_oc + 32;
+    int *s_oc = s_prim + 32, *s_od = s_oc + 32, *s_meta = s_od + 32;
 
     const int n_todo = A.unit_list ? *A.unit_count : A.n_units;
-    const int n_warps = gridDim.x * rysw::kWarps;
+    const int n_teams = gridDim.x * S::kTeams;
     // a queue short for the grid: each unit's groups over several warps
     constexpr int kMaxSlices = (kKetChunk + GW - 1) / GW;
-    const int want = rysw::kItemsPerWarp * n_warps;
+    const int want = rysw::kItemsPerWarp * n_teams;
     int ns = n_todo < want ? (want + n_todo - 1) / max(n_todo, 1) : 1;
     ns = ns > kMaxSlices ? kMaxSlices : ns;
     const int n_items = n_todo * ns;
-    const int grab = max(1, n_items / (n_warps * rysw::kGrabs));
+    const int grab = max(1, n_items / (n_teams * rysw::kGrabs));
 
     // this lane's bra Cartesian (phases B, C)
     const int gl = lane / NBE, el = lane - gl * NBE;
     int ex = 0, ey = 0, ez = 0;
     rys::cart_of<LA, E>(el, &ex, &ey, &ez);
 
-    int left = 0, taken = 0;  // items left of the warp's grab, the next grab's number
-    const int64_t first = (int64_t)(blockIdx.x * rysw::kWarps + wl) * grab;
-    for (int64_t it = first; it < n_items;
-         it = left > 0 ? it + 1
-                       : (A.next ? (int64_t)(n_warps + __shfl_sync(kAll, taken, 0)) * grab
-                                 : it + (int64_t)n_warps * grab - (grab - 1))) {
+    // the items, a grab at a time; the next grab's number comes from the
+    // counter while this one is worked on
+    int left = 0, taken = 0;
+    const auto next_item = [&](int64_t it) -> int64_t {
+        if (left > 0) return it + 1;
+        if (!A.next) return it + (int64_t)n_teams * grab - (grab - 1);
+        if constexpr (TW == 32) {
+            return (int64_t)(n_teams + __shfl_sync(kAll, taken, 0)) * grab;
+        } else {
+            if (lane == 0) s_meta[2] = taken;
+            sync();
+            return (int64_t)(n_teams + s_meta[2]) * grab;  // rewritten only after the next item's barriers
+        }
+    };
+    for (int64_t it = (int64_t)(blockIdx.x * S::kTeams + wl) * grab; it < n_items; it = next_item(it)) {
         if (left == 0) {
             left = grab;
-            if (A.next && lane == 0) taken = atomicAdd(A.next, 1);  // read when the grab is done
+            if (A.next && lane == 0) taken = atomicAdd(A.next, 1);
         }
         --left;
         const int ui = (int)(it / ns), slice = (int)(it - (int64_t)ui * ns);
@@ -183,8 +228,8 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
         const int n_ao = M.n_ao;
         const int kab = bra.nprim;
         const int oa = bra.ao_a, ob = bra.ao_b;
-        int n_list, kcd;
-        {
+        int n_list = 0, kcd = 0;
+        if (lane < 32) {
             const int ik = U.k0 + lane;
             bool on = false;
             PairRec ket{};
@@ -197,7 +242,6 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
             kcd = __shfl_sync(kAll, ket.nprim, 0);  // one degree per ket batch
             if (A.computed && lane == 0 && slice == 0 && n_list)
                 atomicAdd(A.computed + U.launch, (unsigned long long)n_list);
-            if (slice * GW >= n_list) continue;
             if (on) {
                 const int at = __popc(m & ((1u << lane) - 1u));
                 s_prim[at] = ket.prim0;
@@ -208,9 +252,21 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
 #pragma unroll
                 for (int d = 0; d < 3; ++d) s_sep[d * 32 + at] = ket.AB[d];
             }
-            for (int i = lane; i < NAB; i += 32) Dab[i] = __ldg(M.D + (size_t)(oa + i / NB) * n_ao + ob + i % NB);
+            if (TW > 32 && lane == 0) {
+                s_meta[0] = n_list;
+                s_meta[1] = kcd;
+            }
         }
-        __syncwarp();
+        for (int i = lane; i < NAB; i += TW) Dab[i] = __ldg(M.D + (size_t)(oa + i / NB) * n_ao + ob + i % NB);
+        sync();
+        if constexpr (TW > 32) {
+            n_list = s_meta[0];
+            kcd = s_meta[1];
+        }
+        if (slice * GW >= n_list) {
+            sync();  // the lists are read before the next item's
+            continue;
+        }
         const int KNR = kab * kcd * NR;
         double jsum = 0.0;  // sum over this lane's kets of 2 deg sum_cd D_cd [e0|cd]
 
@@ -269,7 +325,7 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
                         }
                     }
                 }
-                __syncwarp();
+                sync();
                 // -- B: this lane's ket row over the entries
                 if (gl < ng) {
                     const int nj = min(CH, KNR - c0);
@@ -296,7 +352,7 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
                             }
                     }
                 }
-                __syncwarp();
+                sync();
             }
 
             // -- C: the ket HRR from the row, to X[g][e][cd]; the bra block's share
@@ -336,7 +392,7 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
                 }
                 jsum += 2.0 * s_deg[at] * s;
             }
-            __syncwarp();
+            sync();
 
             // -- E: the digest of the five ket-dependent blocks
             double pw[3 * (LB + 1)];
@@ -413,18 +469,18 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
                             red_add(M.Jp + (size_t)(oc + c) * n_ao + od + d, 2.0 * deg * jcd);
                         }
 #pragma unroll
-                        for (int a = 0; a < NA; ++a) red[(ci * NK + a) * 32 + lane] = kac[a];
+                        for (int a = 0; a < NA; ++a) red[(ci * NK + a) * TW + lane] = kac[a];
 #pragma unroll
-                        for (int b = 0; b < NB; ++b) red[(ci * NK + NA + b) * 32 + lane] = kbc[b];
+                        for (int b = 0; b < NB; ++b) red[(ci * NK + NA + b) * TW + lane] = kbc[b];
                     }
-                    __syncwarp();
+                    sync();
                     // K_ac and K_bc: the sums over d
 #pragma unroll 1
-                    for (int o = lane; o < GX * CS * BATCH * NK; o += 32) {
+                    for (int o = lane; o < GX * CS * BATCH * NK; o += TW) {
                         const int i = o % NK, r1 = o / NK, ci = r1 % BATCH, r2 = r1 / BATCH, c2 = r2 % CS, g2 = r2 / CS;
                         const int c = c2 + (cb + ci) * CS;
                         if (q0 + g2 < ng && c < NC && cb + ci < CPL) {
-                            const double *rr = red + (ci * NK + i) * 32 + (g2 * CS + c2) * ND;
+                            const double *rr = red + (ci * NK + i) * TW + (g2 * CS + c2) * ND;
                             double s = 0.0;
 #pragma unroll
                             for (int k = 0; k < ND; ++k) s += rr[k];
@@ -433,7 +489,7 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
                             red_add(M.Kp + (size_t)row * n_ao + s_oc[at2] + c, s_deg[at2] * s);
                         }
                     }
-                    __syncwarp();
+                    sync();
                 }
                 if constexpr (CS == 1) {
                     if (on) {
@@ -446,31 +502,42 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
                     }
                 } else {
                     // the residues of c summed over their lanes (the c = 0 lane's adds)
+                    if constexpr (TW > 32) {
+#pragma unroll
+                        for (int i = 0; i < NK; ++i) red[i * TW + lane] = i < NA ? kad[i < NA ? i : 0] : kbd[i < NA ? 0 : i - NA];
+                        sync();
+                    }
 #pragma unroll
                     for (int i = 0; i < NK; ++i) {
-                        double v = i < NA ? kad[i < NA ? i : 0] : kbd[i < NA ? 0 : i - NA];
+                        const double v = i < NA ? kad[i < NA ? i : 0] : kbd[i < NA ? 0 : i - NA];
                         double s = v;
+                        if constexpr (TW == 32) {
 #pragma unroll
-                        for (int k = 1; k < CS; ++k) s += __shfl_down_sync(kAll, v, k * ND);
+                            for (int k = 1; k < CS; ++k) s += __shfl_down_sync(kAll, v, k * ND);
+                        } else if (on && cs == 0) {
+#pragma unroll
+                            for (int k = 1; k < CS; ++k) s += red[i * TW + lane + k * ND];
+                        }
                         if (on && cs == 0)
                             red_add(M.Kp + (size_t)(i < NA ? oa + i : ob + i - NA) * n_ao + od + d, deg * s);
                     }
+                    if constexpr (TW > 32) sync();
                 }
             }
-            __syncwarp();  // X is read before the next group's tables
+            sync();  // X is read before the next group's tables
         }
 
         // -- the bra block: the bra HRR of the lanes' sums, once per item
         red = ws;  // the region is free here
         red[lane] = gl < GW ? jsum : 0.0;
-        __syncwarp();
+        sync();
         if (lane < NBE) {
             double s = red[lane];
 #pragma unroll
             for (int g = 1; g < GW; ++g) s += red[g * NBE + lane];
-            red[32 + lane] = s;
+            red[TW + lane] = s;
         }
-        __syncwarp();
+        sync();
         {
             double pw[3 * (LB + 1)];
             rysw::sep_powers<LB>(bra.AB, pw);
@@ -478,7 +545,7 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
             for (int a = 0; a < NA; ++a)
 #pragma unroll
                 for (int b = 0; b < NB; ++b) {
-                    if (lane != (a * NB + b) % 32) continue;
+                    if (lane != (a * NB + b) % TW) continue;
                     double v = 0.0;
 #pragma unroll
                     for (int kx = 0; kx <= cbs.x[b]; ++kx)
@@ -490,11 +557,11 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
                                               rys::binom(cbs.z[b], kz)) *
                                      pw[cbs.x[b] - kx] * pw[(LB + 1) + cbs.y[b] - ky] *
                                      pw[2 * (LB + 1) + cbs.z[b] - kz] *
-                                     red[32 + es.idx[ca.x[a] + kx][ca.y[a] + ky][ca.z[a] + kz]];
+                                     red[TW + es.idx[ca.x[a] + kx][ca.y[a] + ky][ca.z[a] + kz]];
                     if (v != 0.0) red_add(M.Jp + (size_t)(oa + a) * n_ao + ob + b, v);
                 }
         }
-        __syncwarp();
+        sync();
         red = ws + S::XD;
     }
 }
@@ -503,7 +570,7 @@ __global__ void __launch_bounds__(rysw::kThreads, (rysw::Shape<LA, LB, LC, LD, R
 template <int LA, int LB, int LC, int LD, typename R>
 struct RysWarpOne {
     using S = rysw::Shape<LA, LB, LC, LD, R>;
-    static constexpr int kSmem = rysw::kWarps * S::SMD * (int)sizeof(double);
+    static constexpr int kSmem = S::kTeams * S::SMD * (int)sizeof(double);
     static void attr() {
         static bool done = false;
         if (done) return;
@@ -514,7 +581,7 @@ struct RysWarpOne {
         static const int per_sm = [] {
             attr();
             int n = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_warp_kernel<LA, LB, LC, LD, R>, rysw::kThreads,
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rys_warp_kernel<LA, LB, LC, LD, R>, S::kThreads,
                                                           kSmem);
             return n;
         }();
@@ -522,7 +589,7 @@ struct RysWarpOne {
     }
     static cudaError_t launch(int grid, cudaStream_t st, const KArgs &a) {
         attr();
-        rys_warp_kernel<LA, LB, LC, LD, R><<<grid, rysw::kThreads, kSmem, st>>>(a);
+        rys_warp_kernel<LA, LB, LC, LD, R><<<grid, S::kThreads, kSmem, st>>>(a);
         return cudaGetLastError();
     }
 };

@@ -1,4 +1,4 @@
-// rys_warp_inst.cu -- the warp-autonomous Rys kernel's instantiations, built
+// rys_warp_inst.cu -- the Rys Fock kernel's instantiations, built
 // once per bra class and precision (FJB_RW_PART a class list of rys_warp.h,
 // FJB_RW_FP32 0 or 1) so that they compile in parallel.
 #include "rys_warp.cuh"
