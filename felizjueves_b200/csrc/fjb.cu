@@ -1414,15 +1414,11 @@ void choose_rys(int mode, ClassRun &r) {
         const int per_sm = std::max(1, rys_warp_blocks_per_sm(la, lb, lc, ld, fp32));
         return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
     };
-    const auto take = [&](bool fp32) {
-        // below two units an SM the class's time is one unit's latency: there
-        // the Rys kernel's, which spreads a quartet's primitives over lanes,
-        // is the shorter (3-atom build, all classes: 660 -> 562 us)
-        return mode >= 1 && rys_warp_available(la, lb, lc, ld) &&
-               (mode == 2 || rys_warp_preferred(la, lb, lc, ld, fp32) || r.n_units <= 2 * sm_count());
-    };
-    r.rys64 = take(false);
-    r.rys32 = take(true);
+    // below two units an SM the class's time is one unit's latency: there the
+    // Rys kernel's, which spreads a quartet's primitives over lanes, is the
+    // shorter (3-atom build, all classes: 660 -> 562 us)
+    r.rys64 = r.rys32 = mode >= 1 && rys_warp_available(la, lb, lc, ld) &&
+                        (mode == 2 || rys_warp_preferred(la, lb, lc, ld) || r.n_units <= 2 * sm_count());
     if (r.rys64) r.grid_r64 = grid(false);
     if (r.rys32) r.grid_r32 = grid(true);
 }

@@ -6,8 +6,6 @@
 
 namespace fjb {
 
-bool compiled_available(int la, int lb, int lc, int ld, bool fp32);  // fock_compiled.cu
-
 #define FJB_X(a, b, c, d)                                                         \
     int rys_warp_occ64_##a##b##c##d();                                            \
     int rys_warp_occ32_##a##b##c##d();                                            \
@@ -25,21 +23,21 @@ bool rys_warp_available(int la, int lb, int lc, int ld) {
 }
 
 // Against the register kernel: a short program in registers beats the tables'
-// round trip.  The register kernel's bodies spill where the boundary (bra e x
-// ket f values) grows: measured on a 20-atom cluster of the 64-atom workload's
-// shells (ms, register / warp kernel, FP64): (sp|sf) 1.46 / 2.85, (sp|pp) 1.77
-// / 2.66, (sp|pd) 1.79 / 3.97, (sd|sd) 0.82 / 1.14, (sd|pp) 1.34 / 2.35, (pp|pp)
-// 0.62 / 1.43, but (sd|sf) 3.94 / 1.55, (sd|pd) 5.02 / 2.61, (sp|pf) 4.14 / 2.61,
-// (sp|dd) 1.54 / 1.13, (pp|pd) 4.28 / 2.58, (sf|pp) 3.02 / 2.75; in FP32 the
-// same classes but (sf|pp), whose row in registers is the shorter side, 1.56 / 2.21.
-bool rys_warp_preferred(int la, int lb, int lc, int ld, bool fp32) {
+// round trip; its bodies spill where the boundary (bra e x ket f values of the
+// HGP transfer, e and f from the first, smaller shell's l up) grows.  The line
+// lies between (sd|sd), 100 values, and (sp|dd), 124.  Measured, ms, register /
+// this kernel, FP64: 32-atom cluster of the 64-atom workload's shells, (sp|pd)
+// 5.8 / 13.3, (sp|pp) 5.7 / 10.6, (sp|sf) 4.5 / 9.5, (sd|pp) 4.0 / 6.3, (sd|sd)
+// 2.2 / 3.0, (pp|pp) 2.0 / 4.6; 20 atoms, (sd|pd) 5.0 / 2.5, (pp|pd) 4.3 / 2.3,
+// (sp|pf) 4.1 / 2.6, (sd|sf) 3.9 / 1.5, (sf|pp) 3.0 / 1.7, (sp|dd) 1.5 / 1.1.
+// FP32 falls on the same sides ((sf|pd), 32 atoms, 15.3 / 5.6).
+bool rys_warp_preferred(int la, int lb, int lc, int ld) {
     const auto rows = [](int x, int y) {  // Cartesians of levels x .. x + y
         int n = 0;
         for (int l = x; l <= x + y; ++l) n += (l + 1) * (l + 2) / 2;
         return n;
     };
-    const int e = rows(la, lb), f = rows(lc, ld);
-    return e * f > 100 && !(fp32 && f < e && compiled_available(la, lb, lc, ld, true));
+    return rows(la, lb) * rows(lc, ld) > 100;
 }
 
 int rys_warp_blocks_per_sm(int la, int lb, int lc, int ld, bool fp32) {

@@ -5,8 +5,17 @@
 // short for the grid, a slice of one), the item's computed kets taken GW at a
 // time.  The team is one WARP where the bra's row of Cartesians fits a warp
 // (to dd: 31): then there is no CTA barrier anywhere, the phases are ordered
-// by __syncwarp and the other warps of the SM fill the latencies.  The pf, df
-// and ff bras (34, 52, 74) take a CTA of 128, 64 and 96.  Per group of kets:
+// by __syncwarp and the other warps of the SM fill the latencies.  The longer
+// bras take a CTA (Shape::tw).
+//
+// The larger shell of each pair comes first (LA >= LB, LC >= LD; the plan's
+// records hold the smaller one first, SB and SK turn them): the boundary then
+// spans la <= |e| <= la + lb from the larger l, which is shorter -- 6 e for a
+// ds bra where (sd| has 10, 10 for fs instead of 20, 25 for fp instead of 34 --
+// and the transfers run over the smaller shell's Cartesians.  32-atom build
+// 237 -> 207 ms: (sf|pd) 10.0 -> 6.5, (sf|pp) 8.7 -> 5.1, (pd|pf) 10.1 -> 7.5,
+// though the ps and fs rows lose a little to their shorter rounds ((sp|pf) 7.9
+// -> 8.7, (sd|sf) 4.7 -> 5.5).  Per group of kets:
 //
 //   A  tables: a lane per (ket, primitive quartet x root): the Rys rule at T
 //      (rys_rule.h) and the three axes' 2D integrals I(i, k), the root's
@@ -38,12 +47,12 @@
 // the longer ket side in registers makes it 49 per 15.  A CTA-per-unit kernel
 // of that form spent the rest on barriers and on staging one unit at a time:
 // 32-atom cluster of the 64-atom workload's shells, ms a class, it / this:
-// (pf|df) 16.0 / 6.5, (pf|pf) 13.2 / 5.1, (df|df) 10.2 / 3.0, (df|ff) 9.3 /
-// 2.9; 20 atoms: (pd|pf) 8.7 / 3.8, (sd|pf) 8.0 / 2.4, (pp|pf) 8.1 / 2.3,
-// (sp|ff) 4.4 / 1.3.
+// (pf|df) 16.0 / 5.1, (pf|pf) 13.2 / 4.4, (df|df) 10.2 / 3.1, (df|ff) 9.3 /
+// 2.7; 20 atoms, smaller shells still first: (pd|pf) 8.7 / 3.8, (sd|pf) 8.0 /
+// 2.4, (pp|pf) 8.1 / 2.3, (sp|ff) 4.4 / 1.3.
 //
 // What bounds it: latency and the shared-memory pipe more than FP64.  ncu on
-// (sd|pf) and (pd|df), 14 atoms: FP64 pipe 24 % and 21 %, shared/L1 data pipe
+// (sd|pf) and (pd|df), 14 atoms, smaller shells first: FP64 pipe 24 % and 21 %, shared/L1 data pipe
 // 50 % and 36 %, long scoreboard 4.3 and 2.6 of some 9 and 7 stall cycles an
 // instruction, 16 and 10 warps an SM by registers and shared memory.
 #pragma once
@@ -63,10 +72,20 @@ constexpr int kRedSlots = 12;  // FP64 values a lane parks per reduction round
 template <int LA, int LB, int LC, int LD, typename R>
 struct Shape {
     using S = rys::Shape<LA, LB, LC, LD>;
+    static_assert(LA >= LB && LC >= LD, "the larger shell of a pair first");
     // The team of threads that works on an item: a warp where the bra's row
-    // fits one; for pf (34), df (52) and ff (74) the CTA width that wastes
-    // least of its lanes (3 x 34 of 128, 52 of 64, 74 of 96).
-    static constexpr int TW = S::NBE <= 32 ? 32 : (S::NBE == 34 ? 128 : (S::NBE == 52 ? 64 : 96));
+    // fits one, but five kets of an fp bra (25) on a CTA of 128 unless the ket
+    // row is the 74 doubles of ff: one ket a warp fills few lanes of a table
+    // round ((fp|dd) 4.7 ms / 3.2, FP32 3.9 / 2.5; (fp|fp) 4.4 / 4.4; (fp|ff)
+    // 3.1 / 4.3).  fd (46) takes a CTA of 64 in FP64 and of 96, two kets, in
+    // FP32 ((fd|fd) 3.1 against 3.6, FP32 2.7 against 2.2); ff (74) one of 96.
+    // (32-atom cluster of the 64-atom workload's shells.)
+    static constexpr int tw() {
+        if (S::NBE == 25) return S::NBF * (int)sizeof(R) > 52 * 8 ? 32 : 128;
+        if (S::NBE <= 32) return 32;
+        return S::NBE == 46 && sizeof(R) == 8 ? 64 : 96;
+    }
+    static constexpr int TW = tw();
     static constexpr int kThreads = TW == 32 ? 64 : TW;  // two independent warps, or one team, a CTA
     static constexpr int kTeams = kThreads / TW;
     static constexpr int E = S::E, F = S::F, NR = S::NR;
@@ -99,10 +118,13 @@ struct Shape {
     static constexpr int wd(int n) { return (n * (int)sizeof(R) + 7) / 8; }
     static constexpr int XD = wd(GW * NBE * XS);
     // table entries of each ket a round: a lane per entry; the wider teams'
-    // tables no larger than the rows they make room for afterwards
+    // tables no larger than the rows they make room for afterwards; in FP32 two
+    // entries a lane for the ten kets of a ps bra, whose rounds of three spend
+    // their time between phases ((sp|pf) 6.6 ms / 6.2; FP64 8.7 / 9.0)
     static constexpr int ch() {
         const int most = TW / GW, fit = (XD + RED) / wd(GW * STR);
-        return TW == 32 || fit > most ? most : (fit < 8 ? 8 : fit);
+        if (TW == 32) return GW > 8 && sizeof(R) == 4 ? 2 * most : most;
+        return fit > most ? most : (fit < 8 ? 8 : fit);
     }
     static constexpr int CH = ch();
     static constexpr int TABD = wd(GW * CH * STR);
@@ -164,6 +186,7 @@ __global__ void __launch_bounds__((rysw::Shape<LA, LB, LC, LD, R>::kThreads), (r
     constexpr const rys::CSet<LC, LC> &cc = rys::kCart<LC, LC>;
     constexpr const rys::CSet<LD, LD> &cds = rys::kCart<LD, LD>;
     constexpr double kTwoOverSqrtPi = 1.1283791670955126;
+    constexpr bool SB = LA > LB, SK = LC > LD;  // the record's shells are the other way round
     constexpr unsigned kAll = 0xffffffffu;
 
     extern __shared__ __align__(16) double sm[];
@@ -227,7 +250,8 @@ __global__ void __launch_bounds__((rysw::Shape<LA, LB, LC, LD, R>::kThreads), (r
         const MolCtx M = mol_of(A, U.launch);
         const int n_ao = M.n_ao;
         const int kab = bra.nprim;
-        const int oa = bra.ao_a, ob = bra.ao_b;
+        const int oa = SB ? bra.ao_b : bra.ao_a, ob = SB ? bra.ao_a : bra.ao_b;
+        const double sab[3] = {SB ? -bra.AB[0] : bra.AB[0], SB ? -bra.AB[1] : bra.AB[1], SB ? -bra.AB[2] : bra.AB[2]};
         int n_list = 0, kcd = 0;
         if (lane < 32) {
             const int ik = U.k0 + lane;
@@ -245,12 +269,12 @@ __global__ void __launch_bounds__((rysw::Shape<LA, LB, LC, LD, R>::kThreads), (r
             if (on) {
                 const int at = __popc(m & ((1u << lane) - 1u));
                 s_prim[at] = ket.prim0;
-                s_oc[at] = ket.ao_a;
-                s_od[at] = ket.ao_b;
+                s_oc[at] = SK ? ket.ao_b : ket.ao_a;
+                s_od[at] = SK ? ket.ao_a : ket.ao_b;
                 s_deg[at] = (bra.a == bra.b ? 0.5 : 1.0) * (ket.a == ket.b ? 0.5 : 1.0) *
                             ((LR.diag && ik == U.ib) ? 0.5 : 1.0);
 #pragma unroll
-                for (int d = 0; d < 3; ++d) s_sep[d * 32 + at] = ket.AB[d];
+                for (int d = 0; d < 3; ++d) s_sep[d * 32 + at] = SK ? -ket.AB[d] : ket.AB[d];
             }
             if (TW > 32 && lane == 0) {
                 s_meta[0] = n_list;
@@ -278,13 +302,24 @@ __global__ void __launch_bounds__((rysw::Shape<LA, LB, LC, LD, R>::kThreads), (r
 #pragma unroll 1
             for (int c0 = 0; c0 < KNR; c0 += CH) {
                 // -- A: the tables of CH (primitive quartet, root) entries per ket
-                {
-                    const int g = lane / CH, jl = lane - g * CH, j = c0 + jl;
+#pragma unroll 1
+                for (int i0 = lane; i0 < GW * CH; i0 += TW) {
+                    const int g = i0 / CH, jl = i0 - g * CH, j = c0 + jl;
                     if (g < ng && j < KNR) {
                         const int t = j / NR, r = j - t * NR, ikcd = t / kab, ikab = t - ikcd * kab;
                         double pb[kPrimWords], pk[kPrimWords];
                         rysw::ld_prim(A.prims + bra.prim0 + ikab, pb);
                         rysw::ld_prim(A.prims + s_prim[g0 + g] + ikcd, pk);
+                        // P - A and Q - C of the shells that come first here: the
+                        // records hold them for the other ones, A - B away
+                        if constexpr (SB) {
+#pragma unroll
+                            for (int d = 0; d < 3; ++d) pb[3 + d] -= sab[d];
+                        }
+                        if constexpr (SK) {
+#pragma unroll
+                            for (int d = 0; d < 3; ++d) pk[3 + d] -= s_sep[d * 32 + g0 + g];
+                        }
                         const double p = pb[6], q = pk[6];
                         const double inv = 1.0 / (p + q), rho = p * q * inv;
                         const double qi = q * inv, pi = p * inv;  // rho/p, rho/q
@@ -396,7 +431,7 @@ __global__ void __launch_bounds__((rysw::Shape<LA, LB, LC, LD, R>::kThreads), (r
 
             // -- E: the digest of the five ket-dependent blocks
             double pw[3 * (LB + 1)];
-            rysw::sep_powers<LB>(bra.AB, pw);
+            rysw::sep_powers<LB>(sab, pw);
             const int gx = lane / (ND * CS), rem = lane - gx * (ND * CS), cs = rem / ND, d = rem - cs * ND;
 #pragma unroll 1
             for (int q0 = 0; q0 < ng; q0 += GX) {
@@ -540,7 +575,7 @@ __global__ void __launch_bounds__((rysw::Shape<LA, LB, LC, LD, R>::kThreads), (r
         sync();
         {
             double pw[3 * (LB + 1)];
-            rysw::sep_powers<LB>(bra.AB, pw);
+            rysw::sep_powers<LB>(sab, pw);
 #pragma unroll
             for (int a = 0; a < NA; ++a)
 #pragma unroll

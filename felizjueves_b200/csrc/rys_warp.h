@@ -24,7 +24,7 @@ struct KArgs;
 
 bool rys_warp_available(int la, int lb, int lc, int ld);
 // Whether it is the faster of the class's kernels (rys_warp.cu).
-bool rys_warp_preferred(int la, int lb, int lc, int ld, bool fp32);
+bool rys_warp_preferred(int la, int lb, int lc, int ld);
 int rys_warp_blocks_per_sm(int la, int lb, int lc, int ld, bool fp32);
 cudaError_t rys_warp_launch(int la, int lb, int lc, int ld, bool fp32, int grid, cudaStream_t st, const KArgs &a);
 

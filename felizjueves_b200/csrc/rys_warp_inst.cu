@@ -8,15 +8,15 @@ namespace fjb {
 
 #if FJB_RW_FP32
 #define FJB_X(a, b, c, d)                                                                    \
-    int rys_warp_occ32_##a##b##c##d() { return RysWarpOne<a, b, c, d, float>::occupancy(); } \
+    int rys_warp_occ32_##a##b##c##d() { return RysWarpOne<b, a, d, c, float>::occupancy(); } \
     cudaError_t rys_warp_run32_##a##b##c##d(int grid, cudaStream_t st, const KArgs &k) {     \
-        return RysWarpOne<a, b, c, d, float>::launch(grid, st, k);                           \
+        return RysWarpOne<b, a, d, c, float>::launch(grid, st, k);                           \
     }
 #else
 #define FJB_X(a, b, c, d)                                                                     \
-    int rys_warp_occ64_##a##b##c##d() { return RysWarpOne<a, b, c, d, double>::occupancy(); } \
+    int rys_warp_occ64_##a##b##c##d() { return RysWarpOne<b, a, d, c, double>::occupancy(); } \
     cudaError_t rys_warp_run64_##a##b##c##d(int grid, cudaStream_t st, const KArgs &k) {      \
-        return RysWarpOne<a, b, c, d, double>::launch(grid, st, k);                           \
+        return RysWarpOne<b, a, d, c, double>::launch(grid, st, k);                           \
     }
 #endif
 FJB_RW_PART(FJB_X)

@@ -376,9 +376,10 @@ typedef struct fjb_launch_stat {
 int fjb_launch_stats(const fjb_handle *h, fjb_launch_stat *out, int64_t n);
 
 /* Per class kernel of the last build: its class, device milliseconds
- * (events around the launch on the build's stream), work units and the
- * engine of its FP64 units (0 the HGP interpreter, 1 the register kernel,
- * 2 the Rys kernel). */
+ * (events around the launch on its stream; a build of at most 4 Mi work
+ * units runs its classes side by side, and their times then overlap), work
+ * units and the engine of its FP64 units (0 the HGP interpreter, 1 the
+ * register kernel, 2 the Rys kernel). */
 typedef struct fjb_class_stat {
     int32_t la, lb, lc, ld;
     double ms;
@@ -402,12 +403,11 @@ int fjb_set_class_config32(fjb_handle *h, int la, int lb, int lc, int ld, int th
 /* Which classes run on the Rys kernel -- the Rys quadrature in place of the
  * HGP vertical recurrence, the reference's third engine (rys/roots.py,
  * eri/fock/kernel_frys.py:194), feeding the same HRR and digest.  mode 1
- * (the default): every class without an FP64 register body, and those with
- * one where the Rys kernel measured faster; plus, for the routed build's
- * FP32 units, every class without an FP32 register body.  mode 0: none (the
- * HGP shared-memory interpreter takes them).  mode 2: every class the Rys
- * kernel has.  Applies to the current plan and later ones.  The
- * atomics-free build (FJB_FP64_SCATTER) and the ERI tap keep the HGP
+ * (the default): every class with more than 100 boundary values, and every
+ * class of at most two work units an SM, FP64 and FP32.  mode 2: every class
+ * the Rys kernel has.  mode 0: none (the register kernel, else the HGP
+ * shared-memory interpreter).  Applies to the current plan and later ones.
+ * The atomics-free build (FJB_FP64_SCATTER) and the ERI tap keep the HGP
  * kernels. */
 int fjb_set_rys(fjb_handle *h, int mode);
 
