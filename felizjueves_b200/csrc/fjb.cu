@@ -2871,7 +2871,7 @@ int fjb_coulomb_mixed(fjb_handle *h, const double *D_dev, double *J_dev, double 
     CUDA_OK(h, cudaStreamIsCapturing((cudaStream_t)stream, &cap));
     bool overlap = false;
     CUDA_OK(h, use_side_streams(h->side, 0, cap == cudaStreamCaptureStatusActive, &overlap));
-    if (jengine_build(h->jeng, D_dev, J_dev, tau, threshold, h->boys.p, h->rys.p, h->rys32.p, overlap ? &h->side : nullptr,
+    if (jengine_build(h->jeng, D_dev, J_dev, tau, threshold, h->boys.p, h->rys.p, overlap ? &h->side : nullptr,
                       (cudaStream_t)stream, &err, &nl))
         return fail(h, FJB_E_CUDA, err);
     h->j_launches = nl;

@@ -453,8 +453,7 @@ JEngine *jengine_create(const HostBasis &basis, int device, std::string *err) {
 void jengine_destroy(JEngine *e) { delete e; }
 
 int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, double thr32, const double *boys_tab,
-                  const double *rys_tab, const float *rys_tab32, SideStreams *side, cudaStream_t st, std::string *err,
-                  int *launches) {
+                  const double *rys_tab, SideStreams *side, cudaStream_t st, std::string *err, int *launches) {
     int nl = 0;
     auto check = [&](cudaError_t c, const char *what) {
         if (c == cudaSuccess) return true;
@@ -496,7 +495,7 @@ int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, do
                                  thr32, boys_tab);
             else
                 if (!check(j_rys_launch(lp, lq, cs, JRysArgs{e->recs.p, b0, nb, k0, nk, e->kst.p, e->kdq.p, e->skey.p, e->Dqs.p,
-                                                  e->Jp.p, tau, thr32, rys_tab, rys_tab32}),
+                                                  e->Jp.p, tau, thr32, rys_tab}),
                            "j_rys_kernel"))
                     return -2;
             ++nl;

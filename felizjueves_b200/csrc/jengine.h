@@ -34,12 +34,11 @@ void jengine_destroy(JEngine *e);
 
 // J (n_ao^2, DEVICE, row-major; every element written) from the symmetric
 // density D_dev at threshold tau.  thr32 > 0: the record pairs under it run
-// their R and contraction in FP32.  boys_tab, rys_tab, rys_tab32: the device
+// their R and contraction in FP32.  boys_tab, rys_tab: the device
 // tables.  side: the streams its bra orders run on (null: all on st).
 // *launches receives the kernel launches issued.
 int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, double thr32, const double *boys_tab,
-                  const double *rys_tab, const float *rys_tab32, SideStreams *side, cudaStream_t st, std::string *err,
-                  int *launches);
+                  const double *rys_tab, SideStreams *side, cudaStream_t st, std::string *err, int *launches);
 
 // The host plan of the same sweep, for the bit-exact comparison with the
 // reference's launches(): per record in sweep order its shell pair (a, b),

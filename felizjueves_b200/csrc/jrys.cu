@@ -32,21 +32,17 @@ constexpr int kJRysWarps = 4;
 
 template <int LP, int LQ, typename R>
 __device__ __forceinline__ void j_rys_lane(double T, double rho, double dx, double dy, double dz, int r,
-                                           const double *tab, const float *tab32, const double *dq, R *jp) {
+                                           const double *tab, const double *dq, R *jp) {
     constexpr int L = LP + LQ, NR = L / 2 + 1;
     constexpr double kTwoOverSqrtPi = 1.1283791670955126;
-    R x, w;
-    if constexpr (sizeof(R) == 4) {
-        rys::rule_root_f<NR>(r, T, tab32, &x, &w);
-    } else {
-        rys::rule_root<NR>(r, T, tab, &x, &w);
-    }
-    const R a = (R)(-2.0 * rho) * x;
+    double x, w;
+    rys::rule_root<NR>(r, T, tab, &x, &w);
+    const double a64 = -2.0 * rho * x;
+    const R a = (R)a64, ax = (R)(a64 * dx), ay = (R)(a64 * dy), az = (R)(a64 * dz);
     R X[L + 1], Y[L + 1], Z[L + 1];
     X[0] = (R)1;
     Y[0] = (R)1;
-    Z[0] = (R)(kTwoOverSqrtPi * sqrt(rho)) * w;
-    const R ax = a * (R)dx, ay = a * (R)dy, az = a * (R)dz;
+    Z[0] = (R)(kTwoOverSqrtPi * sqrt(rho) * w);
 #pragma unroll
     for (int t = 0; t < L; ++t) {
         const R ta = (R)t * a;
@@ -81,8 +77,10 @@ __device__ __forceinline__ void j_rys_lane(double T, double rho, double dx, doub
     }
 }
 
-// thr32 > 0: a step of kets whose first (largest) bound is below it runs in
-// FP32 (T, the rule's interval and the J_p sums stay FP64).
+// thr32 > 0: the kets of a chunk of 32 whose first (largest) bound is below it
+// run in FP32, as in j_pq_small_kernel: the products X, Y, Z, D_q and the
+// contraction; T, the rule (which holds the Boys values here) and its factors
+// and the J_p sums stay FP64.  A step that straddles two chunks may run both.
 template <int LP, int LQ>
 __global__ void __launch_bounds__(32 * kJRysWarps) j_rys_kernel(const JRysArgs A) {
     constexpr int L = LP + LQ, NR = L / 2 + 1, NP = nh(LP), NQ = nh(LQ), GK = 32 / NR;
@@ -113,15 +111,15 @@ __global__ void __launch_bounds__(32 * kJRysWarps) j_rys_kernel(const JRysArgs A
                 const double q = Q.w, rho = p * q / (p + q);
                 const double dx = Q.x - Px, dy = Q.y - Py, dz = Q.z - Pz;
                 const double T = rho * (dx * dx + dy * dy + dz * dz);
-                if (A.thr32 > 0.0 && first < A.thr32) {
+                if (A.thr32 > 0.0 && G * A.skey[A.ket0 + ((k0 + g) & ~31)] < A.thr32) {
                     float j32[NP];
 #pragma unroll
                     for (int i = 0; i < NP; ++i) j32[i] = 0.f;
-                    j_rys_lane<LP, LQ, float>(T, rho, dx, dy, dz, r, A.rys_tab, A.rys_tab32, dq + g * NQ, j32);
+                    j_rys_lane<LP, LQ, float>(T, rho, dx, dy, dz, r, A.rys_tab, dq + g * NQ, j32);
 #pragma unroll
                     for (int i = 0; i < NP; ++i) jp[i] += (double)j32[i];
                 } else {
-                    j_rys_lane<LP, LQ, double>(T, rho, dx, dy, dz, r, A.rys_tab, A.rys_tab32, dq + g * NQ, jp);
+                    j_rys_lane<LP, LQ, double>(T, rho, dx, dy, dz, r, A.rys_tab, dq + g * NQ, jp);
                 }
             }
             __syncwarp();

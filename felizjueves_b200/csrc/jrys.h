@@ -40,7 +40,6 @@ struct JRysArgs {
     double *Jp;
     double tau, thr32;
     const double *rys_tab;
-    const float *rys_tab32;
 };
 
 // The classes it is built for: total order above kJSmallL.
