@@ -1853,12 +1853,13 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
     bool overlap = false;
     CUDA_OK(h, use_side_streams(h->side, h->n_units, cap == cudaStreamCaptureStatusActive, &overlap));
     overlap = overlap && !scatter;
-    if (overlap) CUDA_OK(h, h->side.fork(st));
+    Fork fork(overlap ? &h->side : nullptr, st);
+    CUDA_OK(h, fork.begin());
     // the large classes first: their kernels are the longest
     for (size_t rj = 0; rj < h->runs.size(); ++rj) {
         const size_t ri = h->runs.size() - 1 - rj;
         const ClassRun &r = h->runs[ri];
-        const cudaStream_t cs = overlap ? h->side.s[rj % SideStreams::kN] : st;
+        const cudaStream_t cs = fork.at(rj);
         CUDA_OK(h, cudaEventRecordWithFlags(h->cev[ri].first, cs, ev_flags));
         KArgs a{};
         a.computed = h->computed.p;
@@ -1937,7 +1938,7 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
         }
         CUDA_OK(h, cudaEventRecordWithFlags(h->cev[ri].second, cs, ev_flags));
     }
-    if (overlap) CUDA_OK(h, h->side.join(st));
+    CUDA_OK(h, fork.join());
     if (scatter) {
         // the bra blocks' partials in unit order, then each launch's scatter
         // in launch order: J' and K' are the same sums in the same order on
@@ -1963,11 +1964,12 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
                                                h->check_est.p);
         zero_if_kernel<<<cgrid, 256, 0, st>>>(h->Jp32.p, h->Kp32.p, nn, h->check_flag.p);
         launches += 3;
-        if (overlap) CUDA_OK(h, h->side.fork(st));
+        Fork again(overlap ? &h->side : nullptr, st);
+        CUDA_OK(h, again.begin());
         for (size_t rj = 0; rj < h->runs.size(); ++rj) {
             const size_t ri = h->runs.size() - 1 - rj;
             const ClassRun &r = h->runs[ri];
-            const cudaStream_t cs = overlap ? h->side.s[rj % SideStreams::kN] : st;
+            const cudaStream_t cs = again.at(rj);
             KArgs a{};
             a.C = r.dev;
             a.units = h->units.p + r.unit0;
@@ -1989,7 +1991,7 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
             CUDA_OK(h, launch_run(r, cs, a));
             ++launches;
         }
-        if (overlap) CUDA_OK(h, h->side.join(st));
+        CUDA_OK(h, again.join());
     }
     h->built = true;
     CUDA_OK(h, cudaEventRecordWithFlags(h->ev1, st, ev_flags));
@@ -2774,6 +2776,16 @@ int fjb_df_eri3(fjb_handle *h, int aux_shell0, int aux_shell1, double tau, doubl
             if (L.n) launches.push_back(L);
         }
     }
+    for (const Launch &L : launches) {
+        auto key = std::make_tuple(L.la, L.lb, L.lp);
+        auto it = h->e3_dev.find(key);
+        if (it == h->e3_dev.end() || it->second.kab < L.max_kab || it->second.kcd < L.max_kcd) {
+            E3Dev d;
+            if (!eri3_layout(L.la, L.lb, L.lp, L.max_kab, L.max_kcd, &d))
+                return fail(h, FJB_E_LIMIT, "fjb_df_eri3: a class does not fit in shared memory");
+            h->e3_dev.insert_or_assign(key, d);
+        }
+    }
     try {
         CUDA_OK(h, cudaStreamSynchronize(st));  // an earlier call's kernels may still read the units
         h->e3_units.upload(units);
@@ -2787,20 +2799,13 @@ int fjb_df_eri3(fjb_handle *h, int aux_shell0, int aux_shell1, double tau, doubl
     bool overlap = false;  // the classes write disjoint blocks: side by side
     CUDA_OK(h, use_side_streams(h->side, 0, cap == cudaStreamCaptureStatusActive, &overlap));
     std::reverse(launches.begin(), launches.end());  // the largest classes first
-    if (overlap) CUDA_OK(h, h->side.fork(st));
+    Fork fork(overlap ? &h->side : nullptr, st);
+    CUDA_OK(h, fork.begin());
     for (size_t li = 0; li < launches.size(); ++li) {
         const Launch &L = launches[li];
-        const cudaStream_t cs = overlap ? h->side.s[li % SideStreams::kN] : st;
-        auto key = std::make_tuple(L.la, L.lb, L.lp);
-        auto it = h->e3_dev.find(key);
-        if (it == h->e3_dev.end() || it->second.kab < L.max_kab || it->second.kcd < L.max_kcd) {
-            E3Dev d;
-            if (!eri3_layout(L.la, L.lb, L.lp, L.max_kab, L.max_kcd, &d))
-                return fail(h, FJB_E_LIMIT, "fjb_df_eri3: a class does not fit in shared memory");
-            it = h->e3_dev.insert_or_assign(key, d).first;
-        }
+        const cudaStream_t cs = fork.at(li);
         E3Args a{};
-        a.Y = it->second;
+        a.Y = h->e3_dev.at(std::make_tuple(L.la, L.lb, L.lp));
         a.units = h->e3_units.p + L.u0;
         a.n_units = (int)L.n;
         a.pairs = h->e3_pairs.p;
@@ -2818,7 +2823,7 @@ int fjb_df_eri3(fjb_handle *h, int aux_shell0, int aux_shell1, double tau, doubl
         CUDA_OK(h, eri3_launch(L.la, L.lb, L.lp, grid, cs, a));
         if (n_launches) ++*n_launches;
     }
-    if (overlap) CUDA_OK(h, h->side.join(st));
+    CUDA_OK(h, fork.join());
     return FJB_OK;
 }
 
@@ -3457,6 +3462,10 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
     if (precision != FJB_FP64 && precision != FJB_ROUTED)
         return bfail(b, FJB_E_ARG, "fjb_batch_build: precision FJB_FP64 or FJB_ROUTED");
     const double route = precision == FJB_ROUTED ? (threshold > 0.0 ? threshold : 1e-9) : 0.0;
+    if (route > 0.0)
+        for (const ClassRun &r : b->runs)
+            if (!r.has32 && !r.rys32)
+                return bfail(b, FJB_E_LIMIT, "fjb_batch_build: a class has no FP32 kernel for routed units");
     BCUDA_OK(b, cudaSetDevice(b->device));
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned nm = (unsigned)b->mols.size();
@@ -3473,11 +3482,12 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
     const fjb_handle *h0 = b->mols[0];
     bool overlap = false;
     BCUDA_OK(b, use_side_streams(b->side, b->n_units, cap == cudaStreamCaptureStatusActive, &overlap));
-    if (overlap) BCUDA_OK(b, b->side.fork(st));
+    Fork fork(overlap ? &b->side : nullptr, st);
+    BCUDA_OK(b, fork.begin());
     for (size_t rj = 0; rj < b->runs.size(); ++rj) {
         const size_t ri = b->runs.size() - 1 - rj;
         const ClassRun &r = b->runs[ri];
-        const cudaStream_t cs = overlap ? b->side.s[rj % SideStreams::kN] : st;
+        const cudaStream_t cs = fork.at(rj);
         BCUDA_OK(b, cudaEventRecordWithFlags(b->cev[ri].first, cs, ev_flags));
         KArgs a{};
         a.C = r.dev;
@@ -3492,8 +3502,6 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
         a.launch_mol = b->launch_mol.p;
         a.next = b->work_next.p + kCounters * ri;
         if (routed) {
-            if (!r.has32 && !r.rys32)
-                return bfail(b, FJB_E_LIMIT, "fjb_batch_build: a class has no FP32 kernel for routed units");
             int *l32 = b->route_list.p + r.unit0;
             int *l64 = b->route_list.p + b->n_units + r.unit0;
             int *cnt = b->route_counts.p + 4 * ri;
@@ -3522,7 +3530,7 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
         }
         BCUDA_OK(b, cudaEventRecordWithFlags(b->cev[ri].second, cs, ev_flags));
     }
-    if (overlap) BCUDA_OK(b, b->side.join(st));
+    BCUDA_OK(b, fork.join());
     BCUDA_OK(b, cudaEventRecordWithFlags(b->ev1, st, ev_flags));
     const unsigned cx = (unsigned)std::min<size_t>((b->max_nn + 255) / 256, 1024);
     batch_close_kernel<<<dim3(cx, nm), 256, 0, st>>>(b->bm.p);

@@ -481,9 +481,10 @@ int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, do
     if (!check(cudaMemsetAsync(e->Jp.p, 0, e->Jp.n * sizeof(double), st), "memset")) return -2;
     // a bra order's classes add into the same J_p, in turn on one stream; the
     // bra orders run side by side
-    if (side && !check(side->fork(st), "fork")) return -2;
+    Fork fork(side, st);
+    if (!check(fork.begin(), "fork")) return -2;
     for (int lp = kJMaxL; lp >= 0; --lp) {
-        const cudaStream_t cs = side ? side->s[lp] : st;
+        const cudaStream_t cs = fork.at(lp);
         const int b0 = e->L_off[lp], nb = e->L_off[lp + 1] - b0;
         if (nb == 0) continue;
         const int grid = std::max(1, std::min((nb + 3) / 4, sms * 8));
@@ -502,7 +503,7 @@ int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, do
             if (!check(cudaGetLastError(), "j_pq_small_kernel")) return -2;
         }
     }
-    if (side && !check(side->join(st), "join")) return -2;
+    if (!check(fork.join(), "join")) return -2;
     const int pair_grid = std::max(1, std::min((e->n_pairs + 3) / 4, sms * 16));
     j_jab_kernel<<<pair_grid, 128, 0, st>>>(e->recs.p, e->pair_rec0.p, e->pair_nrec.p, e->n_pairs, e->Jp.p, J_dev,
                                             e->n_ao);

@@ -327,17 +327,18 @@ int onee_build(OneElectron *e, const double *charges, const double *coords, int 
         return 1;
     }
     int nl = 0;
-    if (side) ce = side->fork(st);
+    Fork fork(side, st);
+    ce = fork.begin();
     for (int c = kClasses - 1; c >= 0 && ce == cudaSuccess; --c) {
         const int n = e->cls_off[c + 1] - e->cls_off[c];
         if (n == 0) continue;
-        const cudaStream_t cs = side ? side->s[c % SideStreams::kN] : st;
-        kFns[c].fn<<<(n + kOneeThreads - 1) / kOneeThreads, kOneeThreads, 0, cs>>>(e->shells.p, e->ex.p, e->co.p, e->pairs.p + e->cls_off[c], n,
-                                                   e->nuc.p, n_nuc, e->n_ao, S, T, V, H, boys_tab);
+        kFns[c].fn<<<(n + kOneeThreads - 1) / kOneeThreads, kOneeThreads, 0, fork.at(c)>>>(
+            e->shells.p, e->ex.p, e->co.p, e->pairs.p + e->cls_off[c], n, e->nuc.p, n_nuc, e->n_ao, S, T, V, H, boys_tab);
         ++nl;
         ce = cudaGetLastError();
     }
-    if (side && ce == cudaSuccess) ce = side->join(st);
+    const cudaError_t joined = fork.join();
+    if (ce == cudaSuccess) ce = joined;
     if (ce != cudaSuccess) {
         *err = std::string("one-electron launch: ") + cudaGetErrorString(ce);
         return 1;
