@@ -989,22 +989,10 @@ constexpr int kCounters = 8;
 // milliseconds, and the classes' own times (fjb_class_stats) stay apart.
 constexpr int kOverlapUnits = 1 << 22;
 
-// Whether a build on st overlaps: it is small enough, and its side streams
-// are there (made on first use, but not while st is being captured).
-cudaError_t use_side_streams(SideStreams &side, int n_units, bool capturing, bool *use) {
-    *use = n_units <= kOverlapUnits;
-    if (!*use || side.ready) return cudaSuccess;
-    if (capturing) {
-        *use = false;
-        return cudaSuccess;
-    }
-    return side.ensure();
-}
-
 struct fjb_handle {
     int device = 0;
     HostBasis basis;
-    SideStreams side;
+    StreamUser side;
     fjb::JEngine *jeng = nullptr;  // the J-engine, built on first use
     fjb::OneElectron *onee = nullptr;  // the one-electron shell pairs, built on first use
     std::vector<fjb::PairBounds> pair_bounds;  // the plan's D-independent pair bounds, computed once
@@ -1449,6 +1437,7 @@ int finish_create(std::unique_ptr<fjb_handle> &h, fjb_handle **out) {
     }
     if (cudaSetDevice(device) != cudaSuccess) return fail(nullptr, FJB_E_CUDA, "cudaSetDevice failed");
     try {
+        h->side.attach(device);
         static const std::vector<double> boys = boys_table();
         h->boys.upload(boys);
         h->rys.upload(rys_tables_cached().t64);
@@ -1850,9 +1839,7 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
     CUDA_OK(h, cudaStreamIsCapturing(st, &cap));
     const unsigned ev_flags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     CUDA_OK(h, cudaEventRecordWithFlags(h->ev0, st, ev_flags));
-    bool overlap = false;
-    CUDA_OK(h, use_side_streams(h->side, h->n_units, cap == cudaStreamCaptureStatusActive, &overlap));
-    overlap = overlap && !scatter;
+    const bool overlap = h->n_units <= kOverlapUnits && !scatter;
     Fork fork(overlap ? &h->side : nullptr, st);
     CUDA_OK(h, fork.begin());
     // the large classes first: their kernels are the longest
@@ -2020,9 +2007,8 @@ int fjb_fock_build_graph(fjb_handle *h, const double *D_dev, double *J_dev, doub
                       h->g_thr == threshold;
     if (!same) {
         h->drop_graph();
-        bool overlap = false;  // the side streams are made before the capture
-        CUDA_OK(h, use_side_streams(h->side, h->n_units, false, &overlap));
         if (!h->cap_stream) CUDA_OK(h, cudaStreamCreateWithFlags(&h->cap_stream, cudaStreamNonBlocking));
+        if (h->n_units <= kOverlapUnits) CUDA_OK(h, h->side.prepare(h->cap_stream));
         CUDA_OK(h, cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal));
         const int rc = fjb_fock_build(h, D_dev, J_dev, K_dev, G_dev, precision, threshold, h->cap_stream);
         cudaGraph_t graph = nullptr;
@@ -2794,12 +2780,8 @@ int fjb_df_eri3(fjb_handle *h, int aux_shell0, int aux_shell1, double tau, doubl
     }
     CUDA_OK(h, cudaMemsetAsync(out_dev, 0, (size_t)n_ao * n_ao * nb * sizeof(double), st));
     const int sms = sm_count();
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CUDA_OK(h, cudaStreamIsCapturing(st, &cap));
-    bool overlap = false;  // the classes write disjoint blocks: side by side
-    CUDA_OK(h, use_side_streams(h->side, 0, cap == cudaStreamCaptureStatusActive, &overlap));
     std::reverse(launches.begin(), launches.end());  // the largest classes first
-    Fork fork(overlap ? &h->side : nullptr, st);
+    Fork fork(&h->side, st);  // the classes write disjoint blocks: side by side
     CUDA_OK(h, fork.begin());
     for (size_t li = 0; li < launches.size(); ++li) {
         const Launch &L = launches[li];
@@ -2872,11 +2854,7 @@ int fjb_coulomb_mixed(fjb_handle *h, const double *D_dev, double *J_dev, double 
         if (!h->jeng) return fail(h, FJB_E_CUDA, err);
     }
     int nl = 0;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CUDA_OK(h, cudaStreamIsCapturing((cudaStream_t)stream, &cap));
-    bool overlap = false;
-    CUDA_OK(h, use_side_streams(h->side, 0, cap == cudaStreamCaptureStatusActive, &overlap));
-    if (jengine_build(h->jeng, D_dev, J_dev, tau, threshold, h->boys.p, h->rys.p, overlap ? &h->side : nullptr,
+    if (jengine_build(h->jeng, D_dev, J_dev, tau, threshold, h->boys.p, h->rys.p, &h->side,
                       (cudaStream_t)stream, &err, &nl))
         return fail(h, FJB_E_CUDA, err);
     h->j_launches = nl;
@@ -2900,12 +2878,8 @@ int fjb_one_electron(fjb_handle *h, const double *charges, const double *coords,
         if (!h->onee) return fail(h, FJB_E_CUDA, err);
     }
     int nl = 0;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CUDA_OK(h, cudaStreamIsCapturing((cudaStream_t)stream, &cap));
-    bool overlap = false;
-    CUDA_OK(h, use_side_streams(h->side, 0, cap == cudaStreamCaptureStatusActive, &overlap));
     if (onee_build(h->onee, charges, coords, n_nuc, S_dev, T_dev, V_dev, H_dev, h->boys.p,
-                   overlap ? &h->side : nullptr, (cudaStream_t)stream, &err, &nl))
+                   &h->side, (cudaStream_t)stream, &err, &nl))
         return fail(h, FJB_E_CUDA, err);
     return FJB_OK;
 }
@@ -3232,7 +3206,7 @@ extern "C" int fjb_fock_build_noalloc(fjb_handle *h, const double *D_dev, double
 
 struct fjb_batch {
     int device = 0;
-    SideStreams side;
+    StreamUser side;
     double tau = 0.0;
     std::vector<fjb_handle *> mols;
     DevBuf<PairRec> pairs;
@@ -3307,6 +3281,7 @@ int fjb_batch_create(fjb_batch **out, fjb_handle *const *handles, int n) {
     std::vector<int64_t> dsh0, nn0;
     int64_t dsh_total = 0, nn_total = 0;
     try {
+        b->side.attach(b->device);
         for (int m = 0; m < n; ++m) {
             fjb_handle *h = b->mols[m];
             const int P0 = (int)pr.size(), Q0 = (int)n_prims, L0 = (int)lr.size();
@@ -3480,9 +3455,7 @@ int fjb_batch_build(fjb_batch *b, int precision, double threshold, void *stream)
     const unsigned ev_flags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     BCUDA_OK(b, cudaEventRecordWithFlags(b->ev0, st, ev_flags));
     const fjb_handle *h0 = b->mols[0];
-    bool overlap = false;
-    BCUDA_OK(b, use_side_streams(b->side, b->n_units, cap == cudaStreamCaptureStatusActive, &overlap));
-    Fork fork(overlap ? &b->side : nullptr, st);
+    Fork fork(b->n_units <= kOverlapUnits ? &b->side : nullptr, st);
     BCUDA_OK(b, fork.begin());
     for (size_t rj = 0; rj < b->runs.size(); ++rj) {
         const size_t ri = b->runs.size() - 1 - rj;

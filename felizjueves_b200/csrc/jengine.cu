@@ -453,7 +453,7 @@ JEngine *jengine_create(const HostBasis &basis, int device, std::string *err) {
 void jengine_destroy(JEngine *e) { delete e; }
 
 int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, double thr32, const double *boys_tab,
-                  const double *rys_tab, SideStreams *side, cudaStream_t st, std::string *err, int *launches) {
+                  const double *rys_tab, StreamUser *side, cudaStream_t st, std::string *err, int *launches) {
     int nl = 0;
     auto check = [&](cudaError_t c, const char *what) {
         if (c == cudaSuccess) return true;

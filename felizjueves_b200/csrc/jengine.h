@@ -38,7 +38,7 @@ void jengine_destroy(JEngine *e);
 // tables.  side: the streams its bra orders run on (null: all on st).
 // *launches receives the kernel launches issued.
 int jengine_build(JEngine *e, const double *D_dev, double *J_dev, double tau, double thr32, const double *boys_tab,
-                  const double *rys_tab, SideStreams *side, cudaStream_t st, std::string *err, int *launches);
+                  const double *rys_tab, StreamUser *side, cudaStream_t st, std::string *err, int *launches);
 
 // The host plan of the same sweep, for the bit-exact comparison with the
 // reference's launches(): per record in sweep order its shell pair (a, b),

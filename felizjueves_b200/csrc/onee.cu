@@ -310,7 +310,7 @@ OneElectron *onee_create(const HostBasis &basis, int device, std::string *err) {
 void onee_destroy(OneElectron *e) { delete e; }
 
 int onee_build(OneElectron *e, const double *charges, const double *coords, int n_nuc, double *S, double *T,
-               double *V, double *H, const double *boys_tab, SideStreams *side, cudaStream_t st, std::string *err,
+               double *V, double *H, const double *boys_tab, StreamUser *side, cudaStream_t st, std::string *err,
                int *launches) {
     std::vector<double4> nuc(n_nuc);
     for (int q = 0; q < n_nuc; ++q)

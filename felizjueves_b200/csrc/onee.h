@@ -30,7 +30,7 @@ void onee_destroy(OneElectron *e);
 // (charges[k], coords[3k..3k+2]) given on the host.  *launches receives the
 // kernel launches issued.  side: the streams its classes run on (null: st).
 int onee_build(OneElectron *e, const double *charges, const double *coords, int n_nuc, double *S,
-               double *T, double *V, double *H, const double *boys_tab, SideStreams *side, cudaStream_t st,
+               double *T, double *V, double *H, const double *boys_tab, StreamUser *side, cudaStream_t st,
                std::string *err, int *launches);
 
 }  // namespace fjb

@@ -5,7 +5,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <set>
+#include <thread>
 #include <vector>
 
 #include "side_streams.h"
@@ -13,11 +16,14 @@
 using namespace fjb;
 
 // what the stand-in runtime saw
+static std::recursive_mutex g_m;
 static int g_streams, g_events, g_launches;          // live streams and events, launches so far
 static std::map<cudaStream_t, int> g_last;           // a stream's last launch
 static std::map<cudaEvent_t, std::map<cudaStream_t, int>> g_event;  // what an event covers
 static std::map<cudaStream_t, std::map<cudaStream_t, int>> g_seen;  // what a stream has waited for
-static int g_fail_at = -1, g_calls;                  // the call that fails, if any
+static std::map<cudaStream_t, unsigned long long> g_cap;  // the capture a stream is part of
+static std::map<cudaEvent_t, unsigned long long> g_ecap;  // and an event was recorded in
+static int g_fail_at = -1, g_calls;                       // the call that fails, if any
 
 static cudaError_t call() { return g_calls++ == g_fail_at ? cudaErrorUnknown : cudaSuccess; }
 static void need(bool ok, const char *what) {
@@ -25,40 +31,66 @@ static void need(bool ok, const char *what) {
     std::printf("%s\n", what);
     std::exit(1);
 }
+#define LOCKED std::lock_guard<std::recursive_mutex> lock(g_m)
 
 extern "C" {
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+    LOCKED;
     *s = (cudaStream_t)std::malloc(1);
     ++g_streams;
     return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t s) {
+    LOCKED;
+    g_cap.erase(s);
+    g_last.erase(s);
+    g_seen.erase(s);
     std::free(s);
     --g_streams;
     return cudaSuccess;
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+    LOCKED;
     *e = (cudaEvent_t)std::malloc(1);
     ++g_events;
     return cudaSuccess;
 }
 cudaError_t cudaEventDestroy(cudaEvent_t e) {
+    LOCKED;
+    g_event.erase(e);
+    g_ecap.erase(e);
     std::free(e);
     --g_events;
     return cudaSuccess;
 }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    LOCKED;
     if (cudaError_t r = call()) return r;
     g_event[e] = g_seen[s];
     g_event[e][s] = g_last[s];
+    g_ecap[e] = g_cap[s];
     return cudaSuccess;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+    LOCKED;
     if (cudaError_t r = call()) return r;
     for (auto &kv : g_event[e])
         if (kv.second > g_seen[s][kv.first]) g_seen[s][kv.first] = kv.second;
+    need(!g_cap[s] || g_cap[s] == g_ecap[e], "a call outside a capture, or of another, took one of its streams");
+    if (g_ecap[e]) g_cap[s] = g_ecap[e];
     return cudaSuccess;
 }
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus *st, unsigned long long *id,
+                                     cudaGraph_t *, const cudaGraphNode_t **, size_t *) {
+    LOCKED;
+    *id = g_cap[s];
+    *st = *id ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
+}
+static void end_capture(unsigned long long id) {
+    for (auto &kv : g_cap)
+        if (kv.second == id) kv.second = 0;
 }
 
 static void launch(cudaStream_t s) { g_last[s] = ++g_launches; }
@@ -72,8 +104,8 @@ static bool joined(cudaStream_t st, const std::set<cudaStream_t> &used) {
 static cudaStream_t const kCaller = (cudaStream_t)0x10;
 
 // a call that forks, launches n kernels and returns (early: without join)
-static int build(SideStreams *side, int n, bool early, std::set<cudaStream_t> *used) {
-    Fork fork(side, kCaller);
+static int build(StreamUser *user, int n, bool early, std::set<cudaStream_t> *used) {
+    Fork fork(user, kCaller);
     if (fork.begin() != cudaSuccess) return 1;
     for (int i = 0; i < n; ++i) {
         used->insert(fork.at(i));
@@ -84,8 +116,9 @@ static int build(SideStreams *side, int n, bool early, std::set<cudaStream_t> *u
 }
 
 static void test_joins() {
-    SideStreams side;
-    need(side.ensure() == cudaSuccess, "ensure");
+    StreamUser side;
+    side.attach(0);
+    need(side.prepare(kCaller) == cudaSuccess, "prepare");
     for (int n : {0, 1, 5, 20})
         for (bool early : {false, true}) {
             std::set<cudaStream_t> used;
@@ -111,8 +144,87 @@ static void test_joins() {
     need(build(nullptr, 3, false, &used) == 0 && used == std::set<cudaStream_t>{kCaller}, "no side streams: the caller's");
 }
 
+// Many handles: a bounded number of streams, given back with the last handle.
+static void test_bounded() {
+    std::vector<std::unique_ptr<StreamUser>> users;
+    for (int i = 0; i < 512; ++i) {
+        users.push_back(std::make_unique<StreamUser>());
+        users.back()->attach(i % 2);
+        std::set<cudaStream_t> used;
+        need(build(users.back().get(), 10, false, &used) == 0, "build");
+        need(used.size() == SideStreams::kN, "a build did not spread");
+        need(g_streams <= 2 * StreamPool::kSets * SideStreams::kN, "streams grow with the handles");
+    }
+    users.clear();
+    need(g_streams == 0 && g_events == 0, "the pool was not given back");
+}
+
+// Calls that are enqueuing at the same time hold different sets; past the
+// last set a call runs on its own stream.
+static void test_exclusive() {
+    StreamUser u;
+    u.attach(0);
+    std::set<cudaStream_t> firsts;
+    {
+        std::vector<std::unique_ptr<Fork>> f;
+        for (int i = 0; i < StreamPool::kSets + 1; ++i) {
+            f.push_back(std::make_unique<Fork>(&u, kCaller));
+            need(f.back()->begin() == cudaSuccess, "begin");
+            need(firsts.insert(f.back()->at(0)).second, "one set lent twice");
+        }
+        need(f.back()->at(0) == kCaller && f.back()->at(3) == kCaller, "no set free: the caller's stream");
+    }
+    Fork again(&u, kCaller);
+    need(again.begin() == cudaSuccess && again.at(0) != kCaller, "the sets were not given back");
+    again.join();
+    // threads
+    std::vector<std::thread> t;
+    std::map<cudaStream_t, int> busy;
+    for (int i = 0; i < 8; ++i)
+        t.emplace_back([&u, &busy, i] {
+            for (int k = 0; k < 500; ++k) {
+                Fork f(&u, (cudaStream_t)(uintptr_t)(0x100 + i));
+                need(f.begin() == cudaSuccess, "begin");
+                const cudaStream_t s = f.at(0);
+                const bool own = s != (cudaStream_t)(uintptr_t)(0x100 + i);
+                if (own) {
+                    LOCKED;
+                    need(busy[s]++ == 0, "two threads in one set");
+                }
+                std::this_thread::yield();
+                if (own) {
+                    LOCKED;
+                    --busy[s];
+                }
+            }
+        });
+    for (auto &x : t) x.join();
+}
+
+// A set that a capture has joined is its own until the capture ends.
+static void test_capture() {
+    StreamUser u;
+    u.attach(0);
+    need(u.prepare(kCaller) == cudaSuccess, "prepare");
+    const cudaStream_t cs = (cudaStream_t)0x20;
+    g_cap[cs] = 7;
+    const auto set_of = [&u](cudaStream_t st) {
+        Fork f(&u, st);
+        need(f.begin() == cudaSuccess, "begin");
+        return f.at(0);
+    };
+    const cudaStream_t a = set_of(cs), b = set_of(cs);
+    need(a != cs && a == b, "two builds in one capture");
+    need(set_of(kCaller) != a, "a set lent out of a running capture");
+    end_capture(7);
+    need(set_of(kCaller) == a, "the capture's set comes back");
+}
+
 int main() {
     test_joins();
+    test_bounded();
+    test_exclusive();
+    test_capture();
     need(g_streams == 0 && g_events == 0, "streams or events left");
     std::printf("ok\n");
 }
