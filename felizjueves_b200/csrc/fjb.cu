@@ -2008,7 +2008,6 @@ int fjb_fock_build_graph(fjb_handle *h, const double *D_dev, double *J_dev, doub
     if (!same) {
         h->drop_graph();
         if (!h->cap_stream) CUDA_OK(h, cudaStreamCreateWithFlags(&h->cap_stream, cudaStreamNonBlocking));
-        if (h->n_units <= kOverlapUnits) CUDA_OK(h, h->side.prepare(h->cap_stream));
         CUDA_OK(h, cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal));
         const int rc = fjb_fock_build(h, D_dev, J_dev, K_dev, G_dev, precision, threshold, h->cap_stream);
         cudaGraph_t graph = nullptr;

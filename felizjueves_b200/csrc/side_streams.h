@@ -80,21 +80,20 @@ public:
         auto it = devices_.find(device);
         if (--it->second.users == 0) devices_.erase(it);
     }
-    // A set for a call on st, `slot` if that is free; *out null when none is
-    // (or none is made yet and st is being captured).  device is current.
+    // A set for a call on st, `slot` if that is free; *out null when all are
+    // taken.  device is current.
     cudaError_t lend(int device, int slot, cudaStream_t st, SideStreams **out) {
         *out = nullptr;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         unsigned long long id = 0;
         if (cudaError_t e = cudaStreamGetCaptureInfo(st, &cap, &id)) return e;
-        const bool capturing = cap != cudaStreamCaptureStatusNone;
         std::lock_guard<std::mutex> l(m_);
         auto &sets = devices_[device].sets;
         int empty = -1;
         for (int k = 0; k < kSets && !*out && empty != slot; ++k) {
             const int i = (slot + k) % kSets;
             if (!sets[i]) {
-                if (empty < 0 && !capturing) empty = i;
+                if (empty < 0) empty = i;
                 continue;
             }
             if (!sets[i]->lent && usable(*sets[i], cap, id)) *out = sets[i].get();
@@ -102,7 +101,7 @@ public:
         if (!*out && empty >= 0) {
             std::unique_ptr<SideStreams> fresh(new (std::nothrow) SideStreams);
             if (!fresh) return cudaErrorMemoryAllocation;
-            if (cudaError_t e = fresh->make()) return e;
+            if (cudaError_t e = make_uncaptured(*fresh)) return e;
             sets[empty] = std::move(fresh);
             *out = sets[empty].get();
         }
@@ -123,6 +122,14 @@ private:
     std::map<int, Device> devices_;
     unsigned next_slot_ = 0;
 
+    // Making streams and events is not work that a running capture records:
+    // a call captured before any eager one gets its set too.
+    static cudaError_t make_uncaptured(SideStreams &s) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if (cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode)) return e;
+        const cudaError_t e = s.make(), back = cudaThreadExchangeStreamCaptureMode(&mode);
+        return e != cudaSuccess ? e : back;
+    }
     // not part of a capture, or of the caller's own
     static bool usable(const SideStreams &s, cudaStreamCaptureStatus cap, unsigned long long id) {
         cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
@@ -150,13 +157,6 @@ public:
     }
     cudaError_t lend(cudaStream_t st, SideStreams **out) {
         return StreamPool::get().lend(device_, slot_, st, out);
-    }
-    // a set is there for a capture that is about to start
-    cudaError_t prepare(cudaStream_t st) {
-        SideStreams *s = nullptr;
-        const cudaError_t e = lend(st, &s);
-        if (s) StreamPool::get().give_back(s);
-        return e;
     }
 };
 

@@ -23,6 +23,7 @@ static std::map<cudaEvent_t, std::map<cudaStream_t, int>> g_event;  // what an e
 static std::map<cudaStream_t, std::map<cudaStream_t, int>> g_seen;  // what a stream has waited for
 static std::map<cudaStream_t, unsigned long long> g_cap;  // the capture a stream is part of
 static std::map<cudaEvent_t, unsigned long long> g_ecap;  // and an event was recorded in
+static thread_local bool g_relaxed;  // the thread's capture mode
 static int g_fail_at = -1, g_calls;                       // the call that fails, if any
 
 static cudaError_t call() { return g_calls++ == g_fail_at ? cudaErrorUnknown : cudaSuccess; }
@@ -36,6 +37,7 @@ static void need(bool ok, const char *what) {
 extern "C" {
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
     LOCKED;
+    need(g_relaxed, "a stream made in a mode in which a capture refuses it");
     *s = (cudaStream_t)std::malloc(1);
     ++g_streams;
     return cudaSuccess;
@@ -88,6 +90,13 @@ cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus *st
     return cudaSuccess;
 }
 }
+extern "C" cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *m) {
+    LOCKED;
+    const bool was = g_relaxed;
+    g_relaxed = *m == cudaStreamCaptureModeRelaxed;
+    *m = was ? cudaStreamCaptureModeRelaxed : cudaStreamCaptureModeThreadLocal;
+    return cudaSuccess;
+}
 static void end_capture(unsigned long long id) {
     for (auto &kv : g_cap)
         if (kv.second == id) kv.second = 0;
@@ -118,7 +127,6 @@ static int build(StreamUser *user, int n, bool early, std::set<cudaStream_t> *us
 static void test_joins() {
     StreamUser side;
     side.attach(0);
-    need(side.prepare(kCaller) == cudaSuccess, "prepare");
     for (int n : {0, 1, 5, 20})
         for (bool early : {false, true}) {
             std::set<cudaStream_t> used;
@@ -205,9 +213,8 @@ static void test_exclusive() {
 static void test_capture() {
     StreamUser u;
     u.attach(0);
-    need(u.prepare(kCaller) == cudaSuccess, "prepare");
     const cudaStream_t cs = (cudaStream_t)0x20;
-    g_cap[cs] = 7;
+    g_cap[cs] = 7;  // the first call is a captured one: it gets a set all the same
     const auto set_of = [&u](cudaStream_t st) {
         Fork f(&u, st);
         need(f.begin() == cudaSuccess, "begin");
@@ -218,6 +225,7 @@ static void test_capture() {
     need(set_of(kCaller) != a, "a set lent out of a running capture");
     end_capture(7);
     need(set_of(kCaller) == a, "the capture's set comes back");
+    need(!g_relaxed, "the capture mode was not put back");
 }
 
 int main() {

@@ -93,6 +93,33 @@ def test_overlapped_build_order(cuda, lib_built, precision, threshold):
             assert float((a - b).abs().max()) <= (1e-11 if precision == 0 else 1e-8)
 
 
+def test_first_build_captured_overlaps(cuda, lib_built):
+    """A handle's first build inside the caller's own capture: the recorded
+    graph runs its classes side by side, so their times add up to well more
+    than the build's, as an eager build's do."""
+    import torch
+    w = configs.cluster(3, 9)
+    ref = FockEngine(w.basis)
+    ref.plan(w.D, w.tau, w.n_mag, export=False)
+    want = ref.build_host(w.D)
+    del ref
+    eng = FockEngine(w.basis)
+    eng.plan(w.D, w.tau, w.n_mag, export=False)
+    D = torch.tensor(w.D, device=cuda)
+    outs = [torch.zeros_like(D) for _ in range(3)]
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        eng.build(D, J=outs[0], K=outs[1], G=outs[2])
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(outs, want):
+        assert np.abs(a.cpu().numpy() - b).max() <= 1e-11
+    total = eng.last_build_stats()[0]
+    assert sum(r["ms"] for r in eng.class_stats()) > 2.0 * total
+
+
 @pytest.mark.parametrize("atoms", [1, 2, 5])
 def test_j_engine_orders_and_reproduces(cuda, lib_built, oracle_lib, atoms):
     """The J-engine's Rys classes with fewer kets than a warp's step (one
