@@ -2,11 +2,12 @@
 #pragma once
 #include <cuda_runtime_api.h>
 
+#include <array>
 #include <cstddef>
+#include <exception>
 #include <map>
 #include <memory>
 #include <mutex>
-#include <new>
 
 namespace fjb {
 
@@ -19,14 +20,16 @@ struct SideStreams {
     static constexpr int kN = 8;
     cudaStream_t s[kN] = {};
     cudaEvent_t forked = nullptr, joined[kN] = {};
+    int priority = 0;   // the streams' priority
     bool lent = false;  // to a call that is enqueuing (StreamPool)
     SideStreams() = default;
     SideStreams(const SideStreams &) = delete;
     SideStreams &operator=(const SideStreams &) = delete;
-    cudaError_t make() {
+    cudaError_t make(int prio) {
+        priority = prio;
         cudaError_t e = cudaEventCreateWithFlags(&forked, cudaEventDisableTiming);
         for (int i = 0; i < kN && e == cudaSuccess; ++i) {
-            e = cudaStreamCreateWithFlags(&s[i], cudaStreamNonBlocking);
+            e = cudaStreamCreateWithPriority(&s[i], cudaStreamNonBlocking, prio);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&joined[i], cudaEventDisableTiming);
         }
         return e;
@@ -55,14 +58,15 @@ struct SideStreams {
     }
 };
 
-// The process's side streams: at most kSets sets a device, made on first use,
-// however many handles and batches there are, and destroyed with the device's
-// last one.  A set is lent to one call for as long as that call enqueues; what
-// it has enqueued orders the next borrower behind it stream by stream, so
-// callers that build at the same time get sets of their own (their slots
-// differ) and only the fifth shares.  A stream that a capture has joined
-// belongs to it until the capture ends: such a set is lent to calls of the
-// same capture only.
+// The process's side streams: at most kSets sets a device and stream priority
+// (a build's side streams have the priority of the stream it is called on),
+// made on first use, however many handles and batches there are, and destroyed
+// with the device's last one.  A set is lent to one call for as long as that
+// call enqueues; what it has enqueued orders the next borrower behind it
+// stream by stream, so callers that build at the same time get sets of their
+// own (their slots differ) and only the fifth shares.  A stream that a capture
+// has joined belongs to it until the capture ends: such a set is lent to calls
+// of the same capture only.
 class StreamPool {
 public:
     static constexpr int kSets = 4;
@@ -82,13 +86,15 @@ public:
     }
     // A set for a call on st, `slot` if that is free; *out null when all are
     // taken.  device is current.
-    cudaError_t lend(int device, int slot, cudaStream_t st, SideStreams **out) {
+    cudaError_t lend(int device, int slot, cudaStream_t st, SideStreams **out) try {
         *out = nullptr;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         unsigned long long id = 0;
         if (cudaError_t e = cudaStreamGetCaptureInfo(st, &cap, &id)) return e;
+        int prio = 0;
+        if (cudaError_t e = cudaStreamGetPriority(st, &prio)) return e;
         std::lock_guard<std::mutex> l(m_);
-        auto &sets = devices_[device].sets;
+        auto &sets = devices_[device].sets[prio];
         int empty = -1;
         for (int k = 0; k < kSets && !*out && empty != slot; ++k) {
             const int i = (slot + k) % kSets;
@@ -99,14 +105,15 @@ public:
             if (!sets[i]->lent && usable(*sets[i], cap, id)) *out = sets[i].get();
         }
         if (!*out && empty >= 0) {
-            std::unique_ptr<SideStreams> fresh(new (std::nothrow) SideStreams);
-            if (!fresh) return cudaErrorMemoryAllocation;
-            if (cudaError_t e = make_uncaptured(*fresh)) return e;
+            auto fresh = std::make_unique<SideStreams>();
+            if (cudaError_t e = make_uncaptured(*fresh, prio)) return e;
             sets[empty] = std::move(fresh);
             *out = sets[empty].get();
         }
         if (*out) (*out)->lent = true;
         return cudaSuccess;
+    } catch (const std::exception &) {  // out of host memory, at a C entry
+        return cudaErrorMemoryAllocation;
     }
     void give_back(SideStreams *s) {
         std::lock_guard<std::mutex> l(m_);
@@ -116,7 +123,7 @@ public:
 private:
     struct Device {
         int users = 0;
-        std::unique_ptr<SideStreams> sets[kSets];
+        std::map<int, std::array<std::unique_ptr<SideStreams>, kSets>> sets;  // by priority
     };
     std::mutex m_;
     std::map<int, Device> devices_;
@@ -124,10 +131,10 @@ private:
 
     // Making streams and events is not work that a running capture records:
     // a call captured before any eager one gets its set too.
-    static cudaError_t make_uncaptured(SideStreams &s) {
+    static cudaError_t make_uncaptured(SideStreams &s, int prio) {
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         if (cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode)) return e;
-        const cudaError_t e = s.make(), back = cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = s.make(prio), back = cudaThreadExchangeStreamCaptureMode(&mode);
         return e != cudaSuccess ? e : back;
     }
     // not part of a capture, or of the caller's own

@@ -21,6 +21,7 @@ static int g_streams, g_events, g_launches;          // live streams and events,
 static std::map<cudaStream_t, int> g_last;           // a stream's last launch
 static std::map<cudaEvent_t, std::map<cudaStream_t, int>> g_event;  // what an event covers
 static std::map<cudaStream_t, std::map<cudaStream_t, int>> g_seen;  // what a stream has waited for
+static std::map<cudaStream_t, int> g_prio;           // a stream's priority
 static std::map<cudaStream_t, unsigned long long> g_cap;  // the capture a stream is part of
 static std::map<cudaEvent_t, unsigned long long> g_ecap;  // and an event was recorded in
 static thread_local bool g_relaxed;  // the thread's capture mode
@@ -35,16 +36,23 @@ static void need(bool ok, const char *what) {
 #define LOCKED std::lock_guard<std::recursive_mutex> lock(g_m)
 
 extern "C" {
-cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned, int prio) {
     LOCKED;
     need(g_relaxed, "a stream made in a mode in which a capture refuses it");
     *s = (cudaStream_t)std::malloc(1);
+    g_prio[*s] = prio;
     ++g_streams;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamGetPriority(cudaStream_t s, int *prio) {
+    LOCKED;
+    *prio = g_prio[s];
     return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t s) {
     LOCKED;
     g_cap.erase(s);
+    g_prio.erase(s);
     g_last.erase(s);
     g_seen.erase(s);
     std::free(s);
@@ -228,11 +236,25 @@ static void test_capture() {
     need(!g_relaxed, "the capture mode was not put back");
 }
 
+// The side streams have the caller's priority.
+static void test_priority() {
+    StreamUser u;
+    u.attach(0);
+    const cudaStream_t high = (cudaStream_t)0x30;
+    g_prio[high] = -5;
+    for (cudaStream_t st : {kCaller, high, kCaller, high}) {
+        Fork f(&u, st);
+        need(f.begin() == cudaSuccess && f.at(0) != st, "begin");
+        for (int i = 0; i < SideStreams::kN; ++i) need(g_prio[f.at(i)] == g_prio[st], "another priority than the caller's");
+    }
+}
+
 int main() {
     test_joins();
     test_bounded();
     test_exclusive();
     test_capture();
+    test_priority();
     need(g_streams == 0 && g_events == 0, "streams or events left");
     std::printf("ok\n");
 }

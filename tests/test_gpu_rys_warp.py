@@ -93,6 +93,24 @@ def test_overlapped_build_order(cuda, lib_built, precision, threshold):
             assert float((a - b).abs().max()) <= (1e-11 if precision == 0 else 1e-8)
 
 
+def test_build_on_a_priority_stream(cuda, lib_built):
+    """A build on a high-priority stream, between two on a default one."""
+    import torch
+    w = configs.cluster(3, 9)
+    eng = FockEngine(w.basis)
+    eng.plan(w.D, w.tau, w.n_mag, export=False)
+    want = eng.build_host(w.D)
+    D = torch.tensor(w.D, device=cuda)
+    for prio in (0, -5, 0, -5):
+        st = torch.cuda.Stream(priority=prio)
+        st.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(st):
+            got = [m.clone() for m in eng.build(D)]
+        st.synchronize()
+        for a, b in zip(got, want):
+            assert np.abs(a.cpu().numpy() - b).max() <= 1e-11
+
+
 def test_first_build_captured_overlaps(cuda, lib_built):
     """A handle's first build inside the caller's own capture: the recorded
     graph runs its classes side by side, so their times add up to well more

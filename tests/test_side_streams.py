@@ -1,7 +1,7 @@
 """The builds' fork onto side streams (side_streams.h): every way out of a
 call joins it back to the caller's stream; the streams are the process's, as
 many for 512 handles as for four, lent to one call at a time and kept with a
-capture until it ends.  Host logic: the harness runs it against stand-ins for
+capture until it ends; they have the caller's priority.  Host logic: the harness runs it against stand-ins for
 the CUDA calls."""
 
 import os
