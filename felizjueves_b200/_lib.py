@@ -82,6 +82,7 @@ def load():
     L.fjb_set_class_config.argtypes = [vp] + [C.c_int] * 6
     L.fjb_set_class_config32.argtypes = [vp] + [C.c_int] * 6
     L.fjb_set_rys.argtypes = [vp, C.c_int]
+    L.fjb_set_overlap.argtypes = [vp, C.c_int]
     L.fjb_set_route_check.argtypes = [vp, dbl, C.c_int]
     L.fjb_df_jk.argtypes = [vp, vp, i64, i64, vp, vp, vp, vp]
     L.fjb_hjk_plan.argtypes = [vp, vp, dbl, C.c_int, C.c_int]
@@ -130,7 +131,7 @@ EXPORTS = ("fjb_last_error", "fjb_version", "fjb_create", "fjb_destroy", "fjb_n_
            "fjb_fock_build", "fjb_fock_build_host", "fjb_eri_blocks", "fjb_eri_blocks_fp32", "fjb_boys",
            "fjb_last_build_stats", "fjb_launch_stats", "fjb_class_stats",
            "fjb_fma_probe", "fjb_fock_build_noalloc", "fjb_set_class_config", "fjb_set_class_config32",
-           "fjb_set_rys", "fjb_set_route_check", "fjb_route_check_result", "fjb_df_jk", "fjb_df_eri3", "fjb_df_syrk",
+           "fjb_set_rys", "fjb_set_overlap", "fjb_set_route_check", "fjb_route_check_result", "fjb_df_jk", "fjb_df_eri3", "fjb_df_syrk",
            "fjb_hjk_plan", "fjb_hjk_counts", "fjb_hjk_export", "fjb_hjk_keys", "fjb_hjk_k", "fjb_hjk_computed",
            "fjb_batch_create", "fjb_batch_set_densities", "fjb_batch_build", "fjb_batch_stats",
            "fjb_batch_last_error", "fjb_batch_destroy",

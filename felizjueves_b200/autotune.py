@@ -6,7 +6,10 @@ class: the CTA width of its HGP kernel (and, optionally, the chunk of
 primitive quartets a CTA pass holds).  Every candidate is applied to every
 class at once, one build is timed per candidate with CUDA events around each
 class kernel (`FockEngine.class_stats`), the medians over `reps` builds are
-compared class by class, and the winner is set.
+compared class by class, and the winner is set.  The builds timed run every
+class on its HGP kernel and one after another (`FockEngine.serial_hgp`): a
+class that the Rys kernel takes would time that kernel whatever is set, and
+side by side the classes' times would hold one another's.
 """
 
 from __future__ import annotations
@@ -23,33 +26,8 @@ CANDIDATES = ((1, 0), (32, 0), (64, 0), (128, 0), (256, 0), (512, 0), (32, 1), (
 
 
 def autotune(eng, D, candidates=CANDIDATES, reps: int = 1, precision: int = 0) -> dict:
-    import torch
-    classes = [(r["la"], r["lb"], r["lc"], r["ld"]) for r in eng.class_stats()] \
-        if _has_build(eng) else None
-    if classes is None:
-        eng.build(D, precision=precision)
-        torch.cuda.synchronize()
-        classes = [(r["la"], r["lb"], r["lc"], r["ld"]) for r in eng.class_stats()]
-    times: dict[tuple, dict[tuple, float]] = {c: {} for c in classes}
-    for cand in candidates:
-        ok = []
-        for c in classes:
-            try:
-                eng.set_class_config(c, *cand)
-                ok.append(c)
-            except ValueError:
-                pass
-        samples: dict[tuple, list[float]] = {c: [] for c in ok}
-        for _ in range(reps):
-            eng.build(D, precision=precision)
-            torch.cuda.synchronize()
-            for r in eng.class_stats():
-                c = (r["la"], r["lb"], r["lc"], r["ld"])
-                if c in samples:
-                    samples[c].append(r["ms"])
-        for c, v in samples.items():
-            if v:
-                times[c][cand] = float(np.median(v))
+    with eng.serial_hgp():
+        times = _time(eng, D, candidates, reps, eng.set_class_config, precision=precision)
     choice = {}
     for c, t in times.items():
         if not t:
@@ -62,6 +40,34 @@ def autotune(eng, D, candidates=CANDIDATES, reps: int = 1, precision: int = 0) -
                    for c, t in times.items()}}
 
 
+def _time(eng, D, candidates, reps, set_config, **build) -> dict[tuple, dict[tuple, float]]:
+    """Per class, the median class_stats time of each candidate that fits it."""
+    import torch
+
+    def one():
+        eng.build(D, **build)
+        torch.cuda.synchronize()
+        return {(r["la"], r["lb"], r["lc"], r["ld"]): r["ms"] for r in eng.class_stats()}
+
+    times: dict[tuple, dict[tuple, float]] = {c: {} for c in one()}
+    for cand in candidates:
+        samples: dict[tuple, list[float]] = {}
+        for c in times:
+            try:
+                set_config(c, *cand)
+                samples[c] = []
+            except ValueError:
+                pass
+        for _ in range(reps):
+            for c, ms in one().items():
+                if c in samples:
+                    samples[c].append(ms)
+        for c, v in samples.items():
+            if v:
+                times[c][cand] = float(np.median(v))
+    return times
+
+
 CANDIDATES32 = ((32, 0), (64, 0), (128, 0), (256, 0), (512, 0), (32, 1), (64, 1), (128, 1), (256, 1), (512, 1),
                 (128, 2))
 
@@ -69,37 +75,11 @@ CANDIDATES32 = ((32, 0), (64, 0), (128, 0), (256, 0), (512, 0), (32, 1), (64, 1)
 def autotune32(eng, D, candidates=CANDIDATES32, reps: int = 1) -> dict:
     """The routed path's FP32 interpreter, per class: every unit sent to FP32
     (a routing threshold above every bound), one build timed per candidate
-    (threads, slots), the fastest kept per class (classes with an FP32
-    register body run it whatever this sets)."""
-    import torch
+    (threads, slots), the fastest kept per class (it serves the FP32 units of
+    classes that neither the Rys kernel nor an FP32 register body takes)."""
     from . import _lib
-    everything = 1e300
-    times: dict[tuple, dict[tuple, float]] = {}
-    for cand in candidates:
-        classes = [(r["la"], r["lb"], r["lc"], r["ld"]) for r in eng.class_stats()] if times else None
-        if classes is None:
-            eng.build(D, precision=_lib.FJB_ROUTED, threshold=everything)
-            torch.cuda.synchronize()
-            classes = [(r["la"], r["lb"], r["lc"], r["ld"]) for r in eng.class_stats()]
-            times = {c: {} for c in classes}
-        ok = []
-        for c in classes:
-            try:
-                eng.set_class_config32(c, *cand)
-                ok.append(c)
-            except ValueError:
-                pass
-        samples: dict[tuple, list[float]] = {c: [] for c in ok}
-        for _ in range(reps):
-            eng.build(D, precision=_lib.FJB_ROUTED, threshold=everything)
-            torch.cuda.synchronize()
-            for r in eng.class_stats():
-                c = (r["la"], r["lb"], r["lc"], r["ld"])
-                if c in samples:
-                    samples[c].append(r["ms"])
-        for c, v in samples.items():
-            if v:
-                times[c][cand] = float(np.median(v))
+    with eng.serial_hgp():
+        times = _time(eng, D, candidates, reps, eng.set_class_config32, precision=_lib.FJB_ROUTED, threshold=1e300)
     choice = {}
     for c, t in times.items():
         if t:
@@ -108,14 +88,6 @@ def autotune32(eng, D, candidates=CANDIDATES32, reps: int = 1) -> dict:
     return {"choice32": {",".join(map(str, c)): list(v) for c, v in choice.items()},
             "ms32": {",".join(map(str, c)): {f"{k[0]}x{k[1]}": v for k, v in t.items()}
                      for c, t in times.items()}}
-
-
-def _has_build(eng) -> bool:
-    try:
-        eng.class_stats()
-        return True
-    except Exception:
-        return False
 
 
 def apply(eng, table: dict) -> None:

@@ -993,6 +993,7 @@ struct fjb_handle {
     int device = 0;
     HostBasis basis;
     StreamUser side;
+    bool overlap = true;  // class launches side by side (fjb_set_overlap)
     fjb::JEngine *jeng = nullptr;  // the J-engine, built on first use
     fjb::OneElectron *onee = nullptr;  // the one-electron shell pairs, built on first use
     std::vector<fjb::PairBounds> pair_bounds;  // the plan's D-independent pair bounds, computed once
@@ -1839,7 +1840,7 @@ int fjb_fock_build(fjb_handle *h, const double *D_dev, double *J_dev, double *K_
     CUDA_OK(h, cudaStreamIsCapturing(st, &cap));
     const unsigned ev_flags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     CUDA_OK(h, cudaEventRecordWithFlags(h->ev0, st, ev_flags));
-    const bool overlap = h->n_units <= kOverlapUnits && !scatter;
+    const bool overlap = h->overlap && h->n_units <= kOverlapUnits && !scatter;
     Fork fork(overlap ? &h->side : nullptr, st);
     CUDA_OK(h, fork.begin());
     // the large classes first: their kernels are the longest
@@ -2780,7 +2781,7 @@ int fjb_df_eri3(fjb_handle *h, int aux_shell0, int aux_shell1, double tau, doubl
     CUDA_OK(h, cudaMemsetAsync(out_dev, 0, (size_t)n_ao * n_ao * nb * sizeof(double), st));
     const int sms = sm_count();
     std::reverse(launches.begin(), launches.end());  // the largest classes first
-    Fork fork(&h->side, st);  // the classes write disjoint blocks: side by side
+    Fork fork(h->overlap ? &h->side : nullptr, st);  // the classes write disjoint blocks: side by side
     CUDA_OK(h, fork.begin());
     for (size_t li = 0; li < launches.size(); ++li) {
         const Launch &L = launches[li];
@@ -2853,8 +2854,8 @@ int fjb_coulomb_mixed(fjb_handle *h, const double *D_dev, double *J_dev, double 
         if (!h->jeng) return fail(h, FJB_E_CUDA, err);
     }
     int nl = 0;
-    if (jengine_build(h->jeng, D_dev, J_dev, tau, threshold, h->boys.p, h->rys.p, &h->side,
-                      (cudaStream_t)stream, &err, &nl))
+    if (jengine_build(h->jeng, D_dev, J_dev, tau, threshold, h->boys.p, h->rys.p,
+                      h->overlap ? &h->side : nullptr, (cudaStream_t)stream, &err, &nl))
         return fail(h, FJB_E_CUDA, err);
     h->j_launches = nl;
     return FJB_OK;
@@ -2878,7 +2879,7 @@ int fjb_one_electron(fjb_handle *h, const double *charges, const double *coords,
     }
     int nl = 0;
     if (onee_build(h->onee, charges, coords, n_nuc, S_dev, T_dev, V_dev, H_dev, h->boys.p,
-                   &h->side, (cudaStream_t)stream, &err, &nl))
+                   h->overlap ? &h->side : nullptr, (cudaStream_t)stream, &err, &nl))
         return fail(h, FJB_E_CUDA, err);
     return FJB_OK;
 }
@@ -3005,6 +3006,14 @@ int fjb_set_rys(fjb_handle *h, int mode) {
     cudaSetDevice(h->device);
     for (auto &r : h->runs) choose_rys(mode, r);
     h->drop_graph();
+    return FJB_OK;
+}
+
+int fjb_set_overlap(fjb_handle *h, int on) {
+    if (!h) return fail(h, FJB_E_ARG, "null handle");
+    if (on != 0 && on != 1) return fail(h, FJB_E_ARG, "fjb_set_overlap: on is 0 or 1");
+    h->overlap = on != 0;
+    h->drop_graph();  // a captured build holds the old streams
     return FJB_OK;
 }
 

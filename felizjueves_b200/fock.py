@@ -27,6 +27,7 @@ is no CPU path: every number comes from the sm_100a kernels.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from dataclasses import dataclass
 from typing import Iterator
@@ -167,6 +168,7 @@ class FockEngine:
         self._h = h
         self._planned = False
         self._plan_lists = None
+        self._rys_mode, self._overlap = 1, True
 
     def close(self) -> None:
         if getattr(self, "_h", None):
@@ -294,6 +296,27 @@ class FockEngine:
         default) the large classes, 0 or False none (the HGP interpreter),
         2 every class it has."""
         _lib.check(self._L.fjb_set_rys(self._h, int(mode)), self._h)
+        self._rys_mode = int(mode)
+
+    def set_overlap(self, on: bool = True) -> None:
+        """Whether the class kernels run side by side (fjb_set_overlap, the
+        default) or one after another, each `class_stats` time then its
+        kernel's own."""
+        _lib.check(self._L.fjb_set_overlap(self._h, int(bool(on))), self._h)
+        self._overlap = bool(on)
+
+    @contextlib.contextmanager
+    def serial_hgp(self):
+        """Within it, every class on its HGP kernel (register or interpreter)
+        and one after another: what the autotuner sets and times."""
+        mode, overlap = self._rys_mode, self._overlap
+        try:
+            self.set_rys(0)
+            self.set_overlap(False)
+            yield self
+        finally:
+            self.set_rys(mode)
+            self.set_overlap(overlap)
 
     def set_route_check(self, budget: float = 1e-8, stride: int = 32) -> None:
         """The routed build's error-budget check (fjb_set_route_check): a

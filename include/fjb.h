@@ -377,7 +377,8 @@ int fjb_launch_stats(const fjb_handle *h, fjb_launch_stat *out, int64_t n);
 
 /* Per class kernel of the last build: its class, device milliseconds
  * (events around the launch on its stream; a build of at most 4 Mi work
- * units runs its classes side by side, and their times then overlap), work
+ * units runs its classes side by side, and their times then overlap unless
+ * fjb_set_overlap turns that off), work
  * units and the engine of its FP64 units (0 the HGP interpreter, 1 the
  * register kernel, 2 the Rys kernel). */
 typedef struct fjb_class_stat {
@@ -393,11 +394,16 @@ int fjb_class_stats(const fjb_handle *h, fjb_class_stat *out, int64_t n, int64_t
  * holds (0 = sized for occupancy).  Applies to the current plan and to later
  * ones.  This is what the autotuner sets after timing candidates, as the
  * reference's performance/dispatch.py:1-45 picks a batch count from measured
- * medians.  FJB_E_LIMIT if the class does not fit that configuration. */
+ * medians.  It takes effect where the Rys kernel does not run the class
+ * (fjb_set_rys): with mode 1 on the classes of at most 100 boundary values
+ * (those that the Rys kernel has, only with more than two work units an SM),
+ * with mode 0 on every class; and in the atomics-free build.  FJB_E_LIMIT if
+ * the class does not fit that configuration. */
 int fjb_set_class_config(fjb_handle *h, int la, int lb, int lc, int ld, int threads, int slots);
 /* The same for the routed path's FP32 interpreter kernel of a class (used
- * for its FP32 units when the class has no FP32 register body); threads 0
- * and slots 0 restore the FP64 configuration's FP32 twin. */
+ * for its FP32 units when neither the Rys kernel nor an FP32 register body
+ * takes the class); threads 0 and slots 0 restore the FP64 configuration's
+ * FP32 twin. */
 int fjb_set_class_config32(fjb_handle *h, int la, int lb, int lc, int ld, int threads, int slots);
 
 /* Which classes run on the Rys kernel -- the Rys quadrature in place of the
@@ -410,6 +416,13 @@ int fjb_set_class_config32(fjb_handle *h, int la, int lb, int lc, int ld, int th
  * The atomics-free build (FJB_FP64_SCATTER) and the ERI tap keep the HGP
  * kernels. */
 int fjb_set_rys(fjb_handle *h, int mode);
+
+/* Whether this handle's calls run their class kernels side by side on side
+ * streams (on = 1, the default: builds of at most 4 Mi work units, fjb_coulomb,
+ * fjb_one_electron, fjb_df_eri3) or one after another on the caller's stream
+ * (on = 0: fjb_class_stats' times are then each kernel's own, as the autotuner
+ * needs them). */
+int fjb_set_overlap(fjb_handle *h, int on);
 
 /* The batched build: many molecules, each a planned handle (same device,
  * same tau), built together with ONE launch per angular-momentum class --
