@@ -1395,11 +1395,16 @@ int append_shells(fjb_handle *h, const fjb_basis *b, int max_l) {
     return FJB_OK;
 }
 
-// Device staging common to every handle: the Boys table, shell offsets and
-// sizes, the build events.
-// Which kernels a class run's units take from the Rys kernel: mode 0 none;
-// 0 none; 1 the classes without an FP64 (FP32) register body and those where
-// the Rys kernel is the faster; 2 every class it has.
+// Which of a class run's units the Rys kernel takes.  mode 0 none; 2 every
+// class it has; 1 the classes where it is the faster (rys_warp_preferred), and
+// in FP64 the classes of at most two units an SM: there the class's time is one
+// unit's latency, and the Rys kernel's, which spreads a quartet's primitives
+// over lanes, is the shorter (3-atom build, all classes: 660 -> 562 us).  The
+// FP32 units of such small classes stay on their register bodies: the sums over
+// roots and primitives round more than the HGP recurrence's over primitives
+// (all units in FP32, p shells of degree 3: rms error of G 2.7e-7 against
+// 1.7e-7, s and p shells 2.4e-7 / 1.9e-7), for no time (7 atoms routed 3.90 /
+// 3.89 ms).
 void choose_rys(int mode, ClassRun &r) {
     const int la = r.dev.la, lb = r.dev.lb, lc = r.dev.lc, ld = r.dev.ld;
     const auto grid = [&](bool fp32) {
@@ -1407,11 +1412,10 @@ void choose_rys(int mode, ClassRun &r) {
         const int per_sm = std::max(1, rys_warp_blocks_per_sm(la, lb, lc, ld, fp32));
         return (int)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)per_sm * sm_count()));
     };
-    // below two units an SM the class's time is one unit's latency: there the
-    // Rys kernel's, which spreads a quartet's primitives over lanes, is the
-    // shorter (3-atom build, all classes: 660 -> 562 us)
-    r.rys64 = r.rys32 = mode >= 1 && rys_warp_available(la, lb, lc, ld) &&
-                        (mode == 2 || rys_warp_preferred(la, lb, lc, ld) || r.n_units <= 2 * sm_count());
+    const bool has = mode >= 1 && rys_warp_available(la, lb, lc, ld);
+    const bool faster = has && (mode == 2 || rys_warp_preferred(la, lb, lc, ld));
+    r.rys64 = faster || (has && r.n_units <= 2 * sm_count());
+    r.rys32 = faster;
     if (r.rys64) r.grid_r64 = grid(false);
     if (r.rys32) r.grid_r32 = grid(true);
 }
@@ -1430,6 +1434,8 @@ const RysTables &rys_tables_cached() {
     return t;
 }
 
+// Device staging common to every handle: the Boys table, shell offsets and
+// sizes, the build events.
 int finish_create(std::unique_ptr<fjb_handle> &h, fjb_handle **out) {
     const int device = h->device;
     if (device < 0) {  // host-only handle: plans and exports, no builds

@@ -409,9 +409,9 @@ int fjb_set_class_config32(fjb_handle *h, int la, int lb, int lc, int ld, int th
 /* Which classes run on the Rys kernel -- the Rys quadrature in place of the
  * HGP vertical recurrence, the reference's third engine (rys/roots.py,
  * eri/fock/kernel_frys.py:194), feeding the same HRR and digest.  mode 1
- * (the default): every class with more than 100 boundary values, and every
- * class of at most two work units an SM, FP64 and FP32.  mode 2: every class
- * the Rys kernel has.  mode 0: none (the register kernel, else the HGP
+ * (the default): every class with more than 100 boundary values, FP64 and
+ * FP32, and the FP64 units of every class of at most two work units an SM.
+ * mode 2: every class the Rys kernel has.  mode 0: none (the register kernel, else the HGP
  * shared-memory interpreter).  Applies to the current plan and later ones.
  * The atomics-free build (FJB_FP64_SCATTER) and the ERI tap keep the HGP
  * kernels. */

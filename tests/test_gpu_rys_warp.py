@@ -64,6 +64,33 @@ def test_warp_kernel_fp32_tier(cuda, lib_built, name):
     assert 0.0 < np.abs(G32 - G).max() <= 1e-5 * np.abs(G).max()
 
 
+@pytest.mark.parametrize("ls", [(1,), (0, 1)])
+def test_small_classes_keep_their_fp32_bodies(cuda, lib_built, ls):
+    """A system whose classes have a few units each, every unit in FP32: the
+    classes of s and p shells run the FP32 register bodies that they run in
+    large systems, so the default mode's result is mode 0's to FP64 rounding
+    (a Rys build's, mode 2, differs by FP32 rounding)."""
+    from felizjueves_b200 import _lib
+    rng = np.random.default_rng(7)
+    shells = []
+    for c in rng.uniform(0.0, 5.0, (4, 3)):
+        for l in ls:
+            ex = [0.4 * 2.9 ** k for k in range(3)]
+            shells.append(Shell(l, tuple(map(float, c)), ex, [primitive_norm(l, e) / 3 for e in ex]))
+    B = Basis(tuple(shells))
+    D = configs.random_density(rng, B.n_ao, 6)
+    eng = FockEngine(B)
+    eng.plan(D, 1e-12, 4, export=False)
+    eng.set_route_check(0.0)
+    G = {}
+    for mode in (0, 1, 2):
+        eng.set_rys(mode)
+        G[mode] = eng.build_host(D, precision=_lib.FJB_ROUTED, threshold=1e30)[2]
+    scale = np.abs(G[0]).max()
+    assert np.abs(G[2] - G[0]).max() > 1e-9 * scale
+    assert np.abs(G[1] - G[0]).max() <= 1e-12 * scale
+
+
 @pytest.mark.parametrize("precision,threshold", [(0, 0.0), (1, 1e-9)])
 def test_overlapped_build_order(cuda, lib_built, precision, threshold):
     """A small build forks its class launches onto side streams: D written
