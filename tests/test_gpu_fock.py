@@ -212,9 +212,9 @@ def test_routed_build_within_budget(cuda, lib_built, oracle_lib, atoms, seed):
 
 def test_all_fp32_build_at_fp32_accuracy(cuda, lib_built):
     """With a routing threshold above every bound, every unit of every class
-    runs an FP32 kernel (the register bodies and, for the classes without
-    one, the interpreter in FP32): G then agrees with the FP64 build to FP32
-    accuracy, relative to G's size."""
+    runs an FP32 kernel (the Rys kernel's FP32 tier and, for the classes of
+    at most 100 boundary values, the register bodies): G then agrees with the
+    FP64 build to FP32 accuracy, relative to G's size."""
     import torch
     from felizjueves_b200 import _lib, router
     w = configs.cluster(3, 5)
@@ -356,8 +356,8 @@ def test_atomics_free_build_reproducible(cuda, lib_built, oracle_lib, wname, tau
 
 
 def test_fp32_tap_is_the_routed_arithmetic(cuda, lib_built):
-    """fjb_eri_blocks_fp32 (the FP32 recurrences a routed quartet runs)
-    agrees with the FP64 tap to FP32 accuracy measured on the whole sample,
+    """fjb_eri_blocks_fp32 (the HGP recurrences in FP32, what a routed quartet
+    of a register-body class runs) agrees with the FP64 tap to FP32 accuracy measured on the whole sample,
     while single quartets can lose digits to cancellation (the HRR's |AB|^k
     factors): the spread is reported."""
     w = configs.c0()

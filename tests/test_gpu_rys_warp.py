@@ -64,6 +64,32 @@ def test_warp_kernel_fp32_tier(cuda, lib_built, name):
     assert 0.0 < np.abs(G32 - G).max() <= 1e-5 * np.abs(G).max()
 
 
+def test_long_queues_are_taken_several_items_at_a_time(cuda, lib_built):
+    """75 p and 50 f shells: (pp|pf) and (pf|pf) have more than 64 work units
+    a team of the kernel twice over, so its teams take them two or more at a
+    time.  Every quartet once, and the result of the other engines."""
+    rng = np.random.default_rng(1)
+    shells = []
+    for l, n in ((1, 75), (3, 50)):
+        for e, c in zip(rng.uniform(0.4, 1.2, n), rng.uniform(0.0, 2.0, (n, 3))):
+            shells.append(Shell(l, tuple(map(float, c)), [float(e)], [primitive_norm(l, float(e))]))
+    B = Basis(tuple(shells))
+    D = configs.random_density(rng, B.n_ao, 8)
+    eng = FockEngine(B)
+    eng.plan(D, 1e-12, 4, export=False)
+    out = {}
+    for mode in (0, 1):
+        eng.set_rys(mode)
+        out[mode] = (eng.build_host(D), sum(s["computed"] for s in eng.launch_stats()))
+    units = {(r["la"], r["lb"], r["lc"], r["ld"]): r["units"] for r in eng.class_stats()}
+    assert units[1, 1, 1, 3] >= 2 * 64 * 148 * 16  # a warp a team, at most 16 an SM
+    assert units[1, 3, 1, 3] >= 2 * 64 * 148 * 4   # 128 threads a team, at most 4 an SM
+    assert out[0][1] == out[1][1]
+    for a, b in zip(out[1][0], out[0][0]):
+        # sums of 5e7 terms in another order, each to 1e-16 of the largest
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+
+
 @pytest.mark.parametrize("ls", [(1,), (0, 1)])
 def test_small_classes_keep_their_fp32_bodies(cuda, lib_built, ls):
     """A system whose classes have a few units each, every unit in FP32: the
