@@ -980,7 +980,7 @@ cudaError_t launch_run32(const ClassRun &r, cudaStream_t st, const KArgs &a) {
 
 // Launches of one class in one build: FP64, FP32, the sample's FP32 and FP64,
 // the re-run; each has a work counter of its own.
-constexpr int kCounters = 8;
+constexpr int kCounters = 5;
 
 // Builds of at most this many work units overlap their class launches.  Serial
 // / overlapped: 3 atoms of the 64-atom workload's shells (5 k units) 2.2 / 0.56

@@ -15,7 +15,7 @@
 //   segmented radix sort (CUB) of the keys, descending and stable, one
 //                    segment per L: the ket order of launch.py:325.
 //   j_pq_small_kernel<LP, LQ> (lp + lq <= 6: every Hermite index a template
-//   constant, R in registers) / j_pq_kernel<L> (the rest, table-indexed)
+//   constant, R in registers)
 //                    one launch per (bra L, ket L) class: a warp per bra
 //                    record walks the class's sorted kets 32 at a time, one
 //                    lane per ket, and stops after the chunk holding the
@@ -28,14 +28,19 @@
 //                    (-1)^|q| R_{p+q} D_q into its J_p partials; the warp
 //                    reduces them by shuffles and one lane adds them to the
 //                    record's J_p.
+//   j_rys_kernel<LP, LQ> (jrys.cu; lp + lq = 7 .. 12)
+//                    the same launch per class with R as its Rys quadrature: a
+//                    CTA of four warps per bra record, a lane per (ket, root).
+//   The seven bra orders run side by side (side_streams.h); a bra order's
+//   classes add into the same J_p and follow one another on its stream.
 //   j_jab_kernel     warp per unique shell pair: J_ab = sum_records pre
 //                    sum_p E^{ab}_p J_p, written to J[a][b] and mirrored to
 //                    J[b][a]; on a diagonal pair only the lower triangle
 //                    i >= j writes (both positions), so every element of J
 //                    has exactly one writer: no atomics and no zeroing
 //                    (j.py:303-326's scatter).
-// Roofline: j_pq_kernel is FP64-pipe bound (R recursion + NH(LP) x NH(LQ)
-// FMAs per bra-ket record pair); the others are small.
+// Roofline: the two walks are FP64-pipe bound (R or its quadrature's factors,
+// and the contraction with D_q, per bra-ket record pair); the others are small.
 #include "jengine.h"
 
 #include <cub/device/device_segmented_radix_sort.cuh>
@@ -60,9 +65,8 @@ __constant__ int8_t kCart[20][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, 
                                     {0, 2, 0}, {0, 1, 1}, {0, 0, 2}, {3, 0, 0}, {2, 1, 0}, {2, 0, 1}, {1, 2, 0},
                                     {1, 1, 1}, {1, 0, 2}, {0, 3, 0}, {0, 2, 1}, {0, 1, 2}, {0, 0, 3}};
 
-// Hermite indices (t, u, v) of hermite_order(2 * kJMaxL), for R tables.
-constexpr int kNRMax = nh(2 * kJMaxL);  // 455
-__constant__ int8_t kHermR[kNRMax][3];
+// Hermite indices (t, u, v) of hermite_order(kJMaxL).
+__constant__ int8_t kHermR[kNHMax][3];
 
 constexpr int kETab = 4 * 4 * (kJMaxL + 1);  // E[i][j][t], i, j <= 3, t <= 6
 
@@ -420,7 +424,7 @@ JEngine *jengine_create(const HostBasis &basis, int device, std::string *err) {
         return nullptr;
     }
     std::vector<int8_t> herm;
-    for (const auto &h : herm_order(2 * kJMaxL))
+    for (const auto &h : herm_order(kJMaxL))
         for (int d = 0; d < 3; ++d) herm.push_back((int8_t)h[d]);
     std::vector<int> io(e->n_rec);
     std::iota(io.begin(), io.end(), 0);

@@ -19,7 +19,9 @@
 // stream of FMAs into its own J_p partials, summed over lanes and warps once
 // at the end.  The kets' D_q are consecutive in memory; the warp stages them
 // through shared memory with coalesced loads.  FP64-pipe and shared-memory
-// bound: lp, lq = 3, 4 is 390 FMAs a root for 35 shared loads.
+// bound: lp, lq = 3, 4 is 390 FMAs a root for 35 shared loads.  The classes of
+// lp = 6 keep 84 J_p partials a lane and spill (32 bytes stored at (6, 1), 400
+// at (6, 3), 2,116 at (6, 6)), (5, 5) and (5, 6) a little; the other 13 do not.
 #include "jrys.h"
 
 #include "rys_device.cuh"

@@ -15,11 +15,12 @@
 //                                                             (potential.py:1-60)
 // The nuclei are summed in the Hermite basis: R is linear in the charges, so
 // the block's transform -- 100 components of up to 64 terms for (ff) -- runs
-// once per primitive pair, where it ran once per nucleus, and R and Q stay in
+// once per primitive pair, where it ran once per nucleus, and R stays in
 // registers (hermite_r.cuh).  The classes run side by side (side_streams.h):
 // each is a few hundred warps long on its own.
-// Every index is a template constant once the loops unroll, so the tables
-// live in registers (the largest classes spill).  The block is written to
+// Where the transforms unroll (kUnrolled) every index is a template constant
+// and the tables and Q live in registers; (pf), (dd), (df) and (ff) index them
+// at run time, from local memory (3 to 8 KB a thread).  The block is written to
 // (A, B) and mirrored to (B, A); a diagonal pair writes its upper triangle
 // and the mirror only (one_electron.py:90-110), so each matrix is exactly
 // symmetric and every element has one writer: no atomics, no zeroing.

@@ -108,10 +108,7 @@ struct Shape {
     static constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     static constexpr int NAB = NA * NB, NCD = NC * ND;
     static constexpr int NBE = nrange(LA, E), NBF = nrange(LC, F);
-    static constexpr int NCB = HCoefs<LB>::total(), NCK = HCoefs<LD>::total();
-    static constexpr int XS = NBF | 1;  // X row stride, odd: rows start in different banks
-    static constexpr int YS = NCD | 1;
-    static constexpr int N5 = NCD + NA * NC + NA * ND + NB * NC + NB * ND;
+    static constexpr int NCB = HCoefs<LB>::total();
 };
 
 // Dynamic shared memory of one CTA (doubles) when `minb` CTAs share an SM:

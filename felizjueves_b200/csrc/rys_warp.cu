@@ -25,12 +25,15 @@ bool rys_warp_available(int la, int lb, int lc, int ld) {
 // Against the register kernel: a short program in registers beats the tables'
 // round trip; its bodies spill where the boundary (bra e x ket f values of the
 // HGP transfer, e and f from the first, smaller shell's l up) grows.  The line
-// lies between (sd|sd), 100 values, and (sp|dd), 124.  Measured, ms, register /
-// this kernel, FP64: 32-atom cluster of the 64-atom workload's shells, (sp|pd)
-// 5.8 / 13.3, (sp|pp) 5.7 / 10.6, (sp|sf) 4.5 / 9.5, (sd|pp) 4.0 / 6.3, (sd|sd)
-// 2.2 / 3.0, (pp|pp) 2.0 / 4.6; 20 atoms, (sd|pd) 5.0 / 2.5, (pp|pd) 4.3 / 2.3,
-// (sp|pf) 4.1 / 2.6, (sd|sf) 3.9 / 1.5, (sf|pp) 3.0 / 1.7, (sp|dd) 1.5 / 1.1.
-// FP32 falls on the same sides ((sf|pd), 32 atoms, 15.3 / 5.6).
+// lies between (sd|sd), 100 values, and (sp|dd), 124.  32-atom cluster of the
+// 64-atom workload's shells, classes one after another, ms, register / this
+// kernel, FP64: (sp|pd) 5.8 / 13.4, (sp|pp) 5.7 / 10.7, (sp|sf) 4.5 / 9.5,
+// (sd|pp) 4.4 / 6.3, (sd|sd) 2.4 / 3.0, (pp|pp) 2.1 / 4.5; then (sp|dd) 3.8 /
+// 3.0, (sp|pf) 12.0 / 8.8, (pp|pd) 13.7 / 7.4, (sf|pp) 9.8 / 5.1, (sd|pd) 15.7 /
+// 7.3, (sd|sf) 12.1 / 5.5.  In FP32 the two cross a little later -- (sp|dd) 1.9
+// / 2.2, (sp|pf) 4.9 / 6.2, (pp|pd) 5.7 / 5.8, (sf|pp) 3.7 / 3.7, (sd|sf) 4.4 /
+// 4.4, (sd|pd) 6.5 / 5.7 -- and share the line: 1.6 of 163 ms with every unit
+// in FP32.
 bool rys_warp_preferred(int la, int lb, int lc, int ld) {
     const auto rows = [](int x, int y) {  // Cartesians of levels x .. x + y
         int n = 0;

@@ -48,13 +48,14 @@
 // of that form spent the rest on barriers and on staging one unit at a time:
 // 32-atom cluster of the 64-atom workload's shells, ms a class, it / this:
 // (pf|df) 16.0 / 5.1, (pf|pf) 13.2 / 4.4, (df|df) 10.2 / 3.1, (df|ff) 9.3 /
-// 2.7; 20 atoms, smaller shells still first: (pd|pf) 8.7 / 3.8, (sd|pf) 8.0 /
-// 2.4, (pp|pf) 8.1 / 2.3, (sp|ff) 4.4 / 1.3.
+// 2.7; 20 atoms: (pd|pf) 8.7 / 2.2, (sd|pf) 8.0 / 1.8, (pp|pf) 8.1 / 2.0,
+// (sp|ff) 4.4 / 1.1.
 //
 // What bounds it: latency and the shared-memory pipe more than FP64.  ncu on
-// (sd|pf) and (pd|df), 14 atoms, smaller shells first: FP64 pipe 24 % and 21 %, shared/L1 data pipe
-// 50 % and 36 %, long scoreboard 4.3 and 2.6 of some 9 and 7 stall cycles an
-// instruction, 16 and 10 warps an SM by registers and shared memory.
+// (sp|pf), (sd|pf) and (pd|df), 14 atoms: FP64 pipe 32, 29 and 24 %, shared/L1
+// data pipe 68, 74 and 54 %, issue slots 36, 36 and 26 %; of 6.5, 6.3 and
+// 7.5 stall cycles an instruction the long scoreboard has 1.6, 1.1 and 2.6; 12,
+// 12 and 10 warps an SM by registers and shared memory.
 #pragma once
 #include "rys_device.cuh"
 
@@ -131,10 +132,9 @@ struct Shape {
     static constexpr int REGION = TABD > XD + RED ? TABD : XD + RED;
     static constexpr int SMD = REGION + NAB + 32 * 4 + 50;  // + D_ab, the kets' degeneracies, separations, indices
     // CTAs an SM: by shared memory, and by the registers of the ket row (16
-    // warps leave 128 a thread, 12 leave 168, 8 leave 255).  At 16 the rows of
-    // 30 to 34 doubles spill through phase A: (sd|pf) 2.90 ms against 2.39 at
-    // 12, (pp|pf) 2.87 against 2.30; the 16-double row fits, (sf|pd) 3.33
-    // against 3.67 (20-atom cluster of the 64-atom workload's shells).
+    // warps leave 128 a thread, 12 leave 168, 8 leave 255).  The FP64 rows of 25
+    // to 46 doubles want 12: at 16 the 25 of an fp ket spill through phase A
+    // (32-atom build of the 64-atom workload's shells 208.7 ms against 207.3).
     static constexpr int ctas_smem() { return 232448 / (kTeams * SMD * 8 + 1024); }
     static constexpr int warps_regs() {
         const int row = NBF * (int)sizeof(R);
@@ -147,8 +147,8 @@ struct Shape {
     }
 };
 
-// v(y) = sum_{k <= y} C(y, k) SEP^(y-k) x[base + k] for one shell of l = LY:
-// powers of the separation, SEP_d^n at [d * (LY + 1) + n].
+// The powers of a separation that the transfer to a shell of l = LY takes, v(y)
+// = sum_{k <= y} C(y, k) SEP^(y-k) x[base + k]: SEP_d^n at [d * (LY + 1) + n].
 template <int LY>
 __device__ __forceinline__ void sep_powers(const double *sep, double *pw) {
 #pragma unroll

@@ -293,8 +293,8 @@ class FockEngine:
 
     def set_rys(self, mode=1) -> None:
         """Which classes the Rys kernel takes (fjb_set_rys): 1 or True (the
-        default) the large classes, 0 or False none (the HGP interpreter),
-        2 every class it has."""
+        default) the large classes and, in FP64, those of few units, 0 or
+        False none (the HGP kernels), 2 every class it has."""
         _lib.check(self._L.fjb_set_rys(self._h, int(mode)), self._h)
         self._rys_mode = int(mode)
 
@@ -558,8 +558,8 @@ class FockEngine:
 
     def eri_blocks(self, quartets, fp32: bool = False) -> list[np.ndarray]:
         """(ab|cd) of ordered shell quartets, each a (n_a n_b, n_c n_d) array
-        in the reference's eri_block layout; `fp32` with the routed path's
-        FP32 recurrences (what a quartet routed to FP32 contributes)."""
+        in the reference's eri_block layout; `fp32` with the HGP recurrences
+        in FP32 (fjb_eri_blocks_fp32)."""
         import torch
         q = np.ascontiguousarray(np.asarray(quartets, np.int32).reshape(-1, 4))
         off = np.zeros(len(q) + 1, np.int64)

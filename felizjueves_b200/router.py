@@ -243,8 +243,9 @@ def block_max(eng: FockEngine, quartets: np.ndarray) -> np.ndarray:
 
 def block_err(eng: FockEngine, quartets: np.ndarray) -> np.ndarray:
     """max |(ab|cd)_FP32 - (ab|cd)_FP64| of each quartet's block: the FP32
-    tap (fjb_eri_blocks_fp32, the routed path's FP32 recurrences) against
-    the FP64 one, segment maxima on the device."""
+    tap (fjb_eri_blocks_fp32, the HGP recurrences in FP32; a class on the Rys
+    kernel has a smaller error on the workloads' shells) against the FP64
+    one, segment maxima on the device."""
     import torch
     q = np.ascontiguousarray(quartets, np.int32)
     n = len(q)

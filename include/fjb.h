@@ -186,10 +186,14 @@ int fjb_fock_build_host(fjb_handle *h, const double *D_host, double *J_host,
  * Synchronises. */
 int fjb_eri_blocks(fjb_handle *h, const int32_t *quartets, int n, double *out_dev,
                    int64_t *offsets);
-/* The same blocks with the routed path's FP32 recurrences (VRR, boundary and
- * HRR in FP32; Boys and scalars FP64): what a quartet routed to FP32
- * contributes, for measuring its FP32 error (eri/fock/levers/mixed.py's
- * fmixed regions). */
+/* The same blocks with the HGP recurrences in FP32 (VRR, boundary and HRR in
+ * FP32; Boys and scalars FP64): what a routed quartet of a class on an FP32
+ * register body contributes, for measuring its FP32 error
+ * (eri/fock/levers/mixed.py's fmixed regions).  The classes that the Rys kernel
+ * takes (fjb_set_rys) have its rule, tables, boundary and HRR in FP32 instead,
+ * with an error of their own: with every unit in FP32, 3 to 12 atoms of the
+ * 64-atom workload's shells, the rms error of K is 2.2e-7 to 3.2e-7 of it,
+ * where this call's arithmetic gives 7.6e-7 to 8.8e-7. */
 int fjb_eri_blocks_fp32(fjb_handle *h, const int32_t *quartets, int n, double *out_dev,
                         int64_t *offsets);
 
@@ -317,8 +321,9 @@ int fjb_coulomb(fjb_handle *h, const double *D_dev, double *J_dev, double tau, v
 /* The same with the FP32 E/R tier (eri/j_coulomb/levers/mixed.py:101 _f32,
  * as magnitude routing): a chunk of 32 sorted kets whose largest bound
  * I_bra I_ket max|D_q| is below `threshold` runs its R_{tuv} recursion, its
- * signed D_q and the contraction in FP32; T, the Boys values and every J_p
- * sum stay FP64.  threshold 0 is fjb_coulomb. */
+ * signed D_q and the contraction in FP32; T, the Boys values (at total orders
+ * 7 to 12 the Rys rule that R is summed by) and every J_p sum stay FP64.
+ * threshold 0 is fjb_coulomb. */
 int fjb_coulomb_mixed(fjb_handle *h, const double *D_dev, double *J_dev, double tau, double threshold,
                       void *stream);
 /* The atomics-free build's map of plan launch `launch` (plan order): n_el
