@@ -434,8 +434,7 @@ def main():
                      "achieved": round(ach, 3), "peak": round(peak64, 3), "unit": "TFLOP/s",
                      "frac": round(ach / peak64, 4) if peak64 else None, "traffic": None,
                      "traffic_note": "not captured at this size; the kernel is latency- and "
-                                     "shared-memory-bound, its pair records and D read from L2 "
-                                     "(profiles/rys_warp_kernel_cluster14.md)",
+                                     "shared-memory-bound, its pair records and D read from L2",
                      "peak_source": "measured: fjb_fma_probe FP64 FMA chains on this GPU "
                                     "(MEASURED_PEAKS.json has no FP64 figure)",
                      "build_tflops": round(build_tf, 3), "kernel_ms": round(top["ms"], 3),
